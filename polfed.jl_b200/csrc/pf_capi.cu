@@ -375,6 +375,7 @@ int pf_set_step_width(pf_op *op, int dtype, int s, int width) {
     }
     std::lock_guard<std::mutex> lock(op->tune_mu);
     op->tuned_width[std::make_pair(elem, s)] = width;
+    op->pinned_width.insert(std::make_pair(elem, s));
     PF_API_END
 }
 

@@ -8,6 +8,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 #include <stdexcept>
@@ -163,6 +164,7 @@ struct pf_op {
     pf::CsrDesc<double> csr64{};
     pf::CsrDesc<float> csr32{};
     int64_t nnz = 0;
+    int max_row = 0;                  // CSR: entries of the longest row
     // > 0: the real embedding [[A, -B], [B, A]] of a complex Hermitian H = A + iB
     // of this dimension (dim = 2 complex_dim); solved by solve_hermitian
     int64_t complex_dim = 0;
@@ -184,6 +186,8 @@ struct pf_op {
     // autotuned columns-per-thread of the step kernel, keyed by (element bytes, s)
     std::mutex tune_mu;
     std::map<std::pair<int, int>, int> tuned_width;
+    // the (element bytes, s) whose variant the caller pinned: their filters run step by step
+    std::set<std::pair<int, int>> pinned_width;
     // host copies of the defining parameters (for reports and re-creation)
     std::vector<int32_t> bonds;
     std::vector<double> J, Delta, fields, coup, grain;

@@ -1232,14 +1232,6 @@ void launch_colresid(pf_handle *h, cudaStream_t st, int64_t D, int s, const doub
 }
 
 // --------------------------------------------------------------- probes
-__device__ __forceinline__ uint64_t mix64(uint64_t z) {
-    // splitmix64 finaliser (Steele, Lea, Flood 2014)
-    z += 0x9e3779b97f4a7c15ULL;
-    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
-    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
-    return z ^ (z >> 31);
-}
-
 template <typename T>
 __global__ void k_probes(uint32_t D, int R, int kind, uint64_t seed, int col0, T *dst) {
     const uint64_t n = (uint64_t)D * R;
@@ -1247,18 +1239,7 @@ __global__ void k_probes(uint32_t D, int R, int kind, uint64_t seed, int col0, T
          it += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t row = it / R;
         const int c = (int)(it - row * R);
-        const uint64_t key = ((uint64_t)(col0 + c) << 32) ^ row;
-        const uint64_t h1 = mix64(seed ^ mix64(key));
-        double val;
-        if (kind == PF_PROBE_RADEMACHER) {
-            val = (h1 & 1ull) ? 1.0 : -1.0;
-        } else {
-            // Box-Muller on two 53-bit uniforms in (0, 1]
-            const uint64_t h2 = mix64(h1 ^ 0xd1b54a32d192ed03ULL);
-            const double u1 = ((double)(h1 >> 11) + 1.0) * (1.0 / 9007199254740992.0);
-            const double u2 = (double)(h2 >> 11) * (1.0 / 9007199254740992.0);
-            val = sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
-        }
+        const double val = probe_value(kind, seed, row, col0 + c);
         dst[it] = (T)val;
     }
 }

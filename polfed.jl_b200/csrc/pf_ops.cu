@@ -296,6 +296,26 @@ pf_op *create_csr_hermitian(pf_handle *h, int64_t D, int64_t nnz, const int64_t 
     return op;
 }
 
+// Entries of the longest row of a CSR matrix on the device.
+static __global__ void k_csr_longest_row(const int64_t *__restrict__ indptr, int64_t D, int *out) {
+    int most = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x)
+        most = max(most, (int)min(indptr[i + 1] - indptr[i], (int64_t)INT32_MAX));
+    if (most > 0) atomicMax(out, most);
+}
+
+static int csr_longest_row(pf_handle *h, int64_t D, const int64_t *indptr) {
+    int *out = static_cast<int *>(handle_scratch(h, sizeof(int)));
+    int most = 0;
+    PF_CUDA(cudaMemsetAsync(out, 0, sizeof(int), h->stream));
+    k_csr_longest_row<<<grid_for(h, D, 256, 8), 256, 0, h->stream>>>(indptr, D, out);
+    PF_CUDA(cudaGetLastError());
+    count_launches(1);
+    PF_CUDA(cudaMemcpyAsync(&most, out, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    PF_CUDA(cudaStreamSynchronize(h->stream));
+    return most;
+}
+
 pf_op *adopt_csr(pf_handle *h, int64_t D, int64_t nnz, int64_t *dptr, int32_t *didx, double *dv64, float *dv32) {
     pf_op *op = nullptr;
     const int dev = h->device;
@@ -315,6 +335,7 @@ pf_op *adopt_csr(pf_handle *h, int64_t D, int64_t nnz, int64_t *dptr, int32_t *d
     op->csr64 = {dptr, didx, dv64};
     op->csr32 = {dptr, didx, dv32};
     try {
+        op->max_row = csr_longest_row(h, D, dptr);
         build_multi_tables(op);
     } catch (...) {
         delete op;
@@ -344,6 +365,7 @@ pf_op *bind_op(const pf_op *src, pf_handle *h) {
     op->csr64 = src->csr64;
     op->csr32 = src->csr32;
     op->nnz = src->nnz;
+    op->max_row = src->max_row;
     op->complex_dim = src->complex_dim;
     op->d_states = src->d_states;
     op->d_rank_tab = src->d_rank_tab;
@@ -360,6 +382,7 @@ pf_op *bind_op(const pf_op *src, pf_handle *h) {
     {
         std::lock_guard<std::mutex> lock(const_cast<pf_op *>(src)->tune_mu);
         op->tuned_width = src->tuned_width;
+        op->pinned_width = src->pinned_width;
     }
     op->bonds = src->bonds;
     op->J = src->J;

@@ -409,4 +409,25 @@ __device__ __forceinline__ T qsun_diag(const QSunDesc<T> &d, uint32_t row) {
     return dg;
 }
 
+// --------------------------------------------------------------- probes
+__device__ __forceinline__ uint64_t mix64(uint64_t z) {
+    // splitmix64 finaliser (Steele, Lea, Flood 2014)
+    z += 0x9e3779b97f4a7c15ULL;
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
+    return z ^ (z >> 31);
+}
+
+// Entry (row, col) of the random probe block of a seed: +-1 or a standard normal.
+__device__ __forceinline__ double probe_value(int kind, uint64_t seed, uint64_t row, int col) {
+    const uint64_t key = ((uint64_t)col << 32) ^ row;
+    const uint64_t h1 = mix64(seed ^ mix64(key));
+    if (kind == PF_PROBE_RADEMACHER) return (h1 & 1ull) ? 1.0 : -1.0;
+    // Box-Muller on two 53-bit uniforms in (0, 1]
+    const uint64_t h2 = mix64(h1 ^ 0xd1b54a32d192ed03ULL);
+    const double u1 = ((double)(h1 >> 11) + 1.0) * (1.0 / 9007199254740992.0);
+    const double u2 = (double)(h2 >> 11) * (1.0 / 9007199254740992.0);
+    return sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
+}
+
 }  // namespace pf

@@ -125,6 +125,18 @@ struct StageClock {
 static void sync(pf_handle *h) { PF_CUDA(cudaStreamSynchronize(h->stream)); }
 
 // ------------------------------------------------------------ the filter
+// Whether an s-column filter runs whole on chip: it fits and is estimated
+// faster than the step kernels, and the caller asked for neither column slabs
+// nor a step variant of their own.
+template <typename T>
+static bool resident_filter_plan(pf_op *op, int s, ResPlan *plan) {
+    {
+        std::lock_guard<std::mutex> lock(op->tune_mu);
+        if (op->pinned_width.count(std::make_pair((int)sizeof(T), s))) return false;
+    }
+    return op->slab_cols <= 0 && resident_plan<T>(op, s, false, plan);
+}
+
 // Y = sum_k c_k T_k(Htilde) X on RI blocks (ClenshawAlgorithm.jl:12-29).
 // b_k is written in place over b_{k+2}, so two work blocks suffice.
 template <typename T>
@@ -134,20 +146,46 @@ struct Filter {
     std::vector<double> c;
     double a, b;
     DevArray<T> X, Y, A, B;
+    // the whole recurrence in one launch on chip, where a column fits a cluster
+    ResPlan plan;        // set by resident's initialiser
+    bool resident;
+    DevArray<unsigned char> work;
+    DevArray<double> dc;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 
     // io = false: only the two work blocks (the filter engine reads and
     // writes the caller's blocks directly)
     Filter(pf_op *op_, int s_, const std::vector<double> &coeffs, double a_, double b_, bool io = true)
-        : op(op_), s(s_), K((int)coeffs.size() - 1), c(coeffs), a(a_), b(b_) {
+        : op(op_), s(s_), K((int)coeffs.size() - 1), c(coeffs), a(a_), b(b_),
+          resident(io && resident_filter_plan<T>(op_, s_, &plan)) {
         const size_t n = (size_t)op->dim * s;
+        if (resident) {
+            dc.alloc(c.size());
+            work.alloc(plan.work);
+            resident_prepare<T>(op, op->h->stream, plan, work.p);
+            PF_CUDA(cudaMemcpyAsync(dc.p, c.data(), c.size() * sizeof(double), cudaMemcpyHostToDevice, op->h->stream));
+            return;
+        }
         if (io) {
             X.alloc(n);
             Y.alloc(n);
         }
         if (K >= 1) A.alloc(n);
         if (K >= 2) B.alloc(n);
+    }
+    // the fixed input and output blocks (a resident filter allocates them on first use)
+    T *x() {
+        if (!X.p) X.alloc((size_t)op->dim * s);
+        return X.p;
+    }
+    T *y() {
+        if (!Y.p) Y.alloc((size_t)op->dim * s);
+        return Y.p;
+    }
+    // Yo = filter of Xi, elements (i, c) at i * xr + c * xc and i * yr + c * yc
+    void run_resident(cudaStream_t st, const T *Xi, int64_t xr, int64_t xc, T *Yo, int64_t yr, int64_t yc) {
+        resident_filter<T>(op, st, plan, work.p, s, K, dc.p, a, b, Xi, xr, xc, Yo, yr, yc);
     }
     ~Filter() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -195,6 +233,10 @@ struct Filter {
     }
     // Capture the K+1 launches once; every later application is one graph launch.
     void run(cudaStream_t st) {
+        if (resident) {
+            run_resident(st, x(), s, 1, y(), s, 1);
+            return;
+        }
         if (!exec) {
             PF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
             const int64_t before = thread_launches();  // captured launches do not execute
@@ -231,6 +273,32 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
     PF_CHECK(N >= 1 && R >= 1, PF_ERR_INVALID, "KPM needs N >= 1 and R >= 1");
     std::vector<double> mu(N, 0.0);
     const int M = (N - 1 + 1) / 2;  // steps: ceil((N-1)/2)
+    // one on-chip recurrence per probe where a column fits a cluster (its dot
+    // partials, 2^(clog + 4) bytes a probe and step, in at most 1 GB)
+    ResPlan plan;
+    if ((int64_t)(M + 1) * R <= ((int64_t)1 << 22) && resident_plan<T>(op, R, true, &plan)) {
+        DevArray<unsigned char> work(plan.work);
+        DevArray<double> parts((size_t)2 * (M + 1) * R << plan.clog), rd((size_t)2 * (M + 1) * R);
+        std::vector<double> hr((size_t)2 * (M + 1) * R);
+        resident_prepare<T>(op, st, plan, work.p);
+        resident_kpm<T>(op, st, plan, work.p, M, R, a, b, probes_cm, ldp, kind, seed, parts.p, rd.p);
+        PF_CUDA(cudaMemcpyAsync(hr.data(), rd.p, hr.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        sync(h);
+        for (int c = 0; c < R; ++c) {
+            const double m0 = hr[c];
+            mu[0] += m0;
+            if (M < 1) continue;
+            const double m1 = hr[(size_t)3 * R + c];   // <v1, v0>
+            if (N > 1) mu[1] += m1;
+            for (int n = 0; n < M; ++n) {
+                if (2 * n + 2 < N) mu[2 * n + 2] += 2.0 * hr[(size_t)2 * (n + 1) * R + c] - m0;
+                if (n >= 1 && 2 * n + 1 < N) mu[2 * n + 1] += 2.0 * hr[((size_t)2 * (n + 1) + 1) * R + c] - m1;
+            }
+        }
+        for (double &m : mu) m *= (double)D / (double)R;
+        if (block_matvecs) *block_matvecs += (int64_t)R * M;
+        return mu;
+    }
     const int RB = std::min(64, R);
     DevArray<T> v0((size_t)D * RB), v1((size_t)D * RB);
     DevArray<double> dots((size_t)std::max(M, 1) * 2 * RB), n0(RB), scl(RB);
@@ -1164,6 +1232,10 @@ static int refine_fp64(pf_op *op, const std::vector<double> &coeffs, double a, d
             const int wc = std::min(wmax, m - c0);
             auto &f = filters[wc];
             if (!f) f.reset(new Filter<double>(op, wc, coeffs, a, b));
+            if (f->resident) {
+                f->run_resident(st, Psi.p + c0, m, 1, W.p + c0, m, 1);
+                continue;
+            }
             PF_CUDA(cudaMemcpy2DAsync(f->X.p, (size_t)wc * sizeof(double), Psi.p + c0, (size_t)m * sizeof(double),
                                       (size_t)wc * sizeof(double), (size_t)D, cudaMemcpyDeviceToDevice, st));
             f->run(st);
@@ -1335,12 +1407,22 @@ void op_filter(pf_op *op, int dtype, double a, double b, int K, const double *co
     const int64_t D = op->dim;
     if (dtype == PF_F64) {
         Filter<double> f(op, s, c, a, b);
+        if (f.resident) {
+            f.run_resident(st, (const double *)X, 1, ldx, (double *)Y, 1, ldy);
+            sync(op->h);
+            return;
+        }
         launch_cm_to_ri<double, double>(st, D, s, (const double *)X, ldx, f.X.p);
         f.enqueue(st);
         launch_ri_to_cm<double, double>(st, D, s, f.Y.p, (double *)Y, ldy);
         sync(op->h);
     } else if (dtype == PF_F32) {
         Filter<float> f(op, s, c, a, b);
+        if (f.resident) {
+            f.run_resident(st, (const float *)X, 1, ldx, (float *)Y, 1, ldy);
+            sync(op->h);
+            return;
+        }
         launch_cm_to_ri<float, float>(st, D, s, (const float *)X, ldx, f.X.p);
         f.enqueue(st);
         launch_ri_to_cm<float, float>(st, D, s, f.Y.p, (float *)Y, ldy);
@@ -1532,7 +1614,15 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     LanczosOut out;
     double stage[6] = {0, 0, 0, 0, 0, 0};
     const int fdtype = P->precision == PF_PREC_FP64 ? PF_F64 : PF_F32;
-    if (P->autotune) {
+    // A handle working for a request pool hands its filters to the pool's
+    // engine, which batches the Clenshaw steps of every solve in flight into
+    // shared launches; otherwise the filter runs whole on chip where it can, or
+    // is this solve's own CUDA graph of steps, whose kernel is tuned.
+    pf_engine *eng = (h->engine && multi_eligible(op, fdtype)) ? h->engine : nullptr;
+    ResPlan onchip;
+    const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, &onchip)
+                                                 : resident_filter_plan<float>(op, s, &onchip));
+    if (P->autotune && steps) {
         bool have;
         {
             std::lock_guard<std::mutex> lock(op->tune_mu);
@@ -1540,16 +1630,16 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
         }
         if (!have && !cached_step_variant(op, s, fdtype)) autotune_step(op, s, fdtype, nullptr);
     }
-    // A handle working for a request pool hands its filters to the pool's
-    // engine, which batches the Clenshaw steps of every solve in flight into
-    // shared launches; otherwise the filter is this solve's own CUDA graph.
-    pf_engine *eng = (h->engine && multi_eligible(op, fdtype)) ? h->engine : nullptr;
     const int ew = engine_width(op, s, fdtype == PF_F64 ? 8 : 4);
     if (P->precision == PF_PREC_FP64) {
         Filter<double> filt(op, s, coeffs, a, b, eng == nullptr);
         BlockMap fmap = [&](const double *X, double *Y) {
             if (eng) {
                 engine_filter(eng, op, st, 8, s, ew, coeffs, a, b, (void *)X, Y, filt.A.p, filt.B.p);
+                return;
+            }
+            if (filt.resident) {
+                filt.run_resident(st, X, s, 1, Y, s, 1);
                 return;
             }
             PF_CUDA(cudaMemcpyAsync(filt.X.p, X, (size_t)D * s * sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -1564,12 +1654,12 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
         // last target is the filter ratio P(lambda_{2 nev}) / P(lambda_{nev})
         const int guard = std::max(s, nev);
         {
-            Filter<float> filt(op, s, coeffs, a, b);
+            Filter<float> filt(op, s, coeffs, a, b, eng == nullptr);
             BlockMap fmap = [&](const double *X, double *Y) {
-                launch_ri_to_cm<double, float>(st, (int64_t)D * s, 1, X, filt.X.p, (int64_t)D * s);
-                if (eng) engine_filter(eng, op, st, 4, s, ew, coeffs, a, b, filt.X.p, filt.Y.p, filt.A.p, filt.B.p);
+                launch_ri_to_cm<double, float>(st, (int64_t)D * s, 1, X, filt.x(), (int64_t)D * s);
+                if (eng) engine_filter(eng, op, st, 4, s, ew, coeffs, a, b, filt.x(), filt.y(), filt.A.p, filt.B.p);
                 else filt.run(st);
-                launch_ri_to_cm<float, double>(st, (int64_t)D * s, 1, filt.Y.p, Y, (int64_t)D * s);
+                launch_ri_to_cm<float, double>(st, (int64_t)D * s, 1, filt.y(), Y, (int64_t)D * s);
             };
             lanczos(op, s, nev, (int)maxdim, P->tol, P->eigentol, P->which, P->reorth_passes, xri.p, fmap, out, stage,
                     refine ? guard : -1, P->host_qr != 0);

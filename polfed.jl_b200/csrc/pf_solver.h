@@ -93,6 +93,37 @@ void blk_update(cudaStream_t st, int64_t D, int s, double *r, const double *V, c
 void small_chol(cudaStream_t st, const double *G, int s, double *R, const double *rtot_in, double *rtot_out,
                 int *flag);
 
+// whole recurrences on chip (pf_resident.cu): a filter or the KPM recurrence
+// of every column in one launch, each column (or few) in one thread-block cluster
+struct ResPlan {
+    int clog = 0;         // log2 of the CTAs per cluster
+    int cols = 1;         // columns per cluster
+    int threads = 0;
+    int rows = 0, groups = 0, list_smem = 0, x_smem = 0, diag_smem = 0;   // operators with neighbour lists
+    size_t smem = 0;
+    size_t work = 0;      // bytes of device workspace
+    double us = 0, busy_us = 0;   // estimated time of a step of one cluster, and of that the time its SMs are busy
+    const void *kern = nullptr;
+};
+// The plan for ncol columns of the operator; false: none (a column does not fit a cluster).
+template <typename T>
+bool resident_plan(const pf_op *op, int ncol, bool kpm, ResPlan *plan);
+// Fills the workspace (plan.work bytes) for the operator; once per workspace.
+template <typename T>
+void resident_prepare(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work);
+// Y = sum_k coef[k] T_k(Htilde) X; element (i, c) of X at i * xr + c * xc, of
+// Y at i * yr + c * yc; coef: K + 1 coefficients in device memory.
+template <typename T>
+void resident_filter(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work, int s, int K, const double *coef,
+                     double a, double b, const T *X, int64_t xr, int64_t xc, T *Y, int64_t yr, int64_t yc);
+// M doubling steps from R probes (column-major, or drawn and normalised from
+// the seed when null): dots[0 * R + c] = <v_0, v_0>, and for step n = 1..M
+// dots[2 n * R + c] = <v_n, v_n>, dots[(2 n + 1) * R + c] = <v_n, v_{n-1}>.
+// part: 2 (M + 1) R 2^clog doubles; dots: 2 (M + 1) R.
+template <typename T>
+void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work, int M, int R, double a, double b,
+                  const T *probes, int64_t ldp, int kind, uint64_t seed, double *part, double *dots);
+
 // filter engine (pf_engine.cu): one step launch for every filter in flight
 void build_multi_tables(pf_op *op);
 bool multi_eligible(const pf_op *op, int dtype);
