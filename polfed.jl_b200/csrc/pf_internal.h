@@ -267,6 +267,15 @@ bool cached_step_variant(pf_op *op, int s, int dtype);
 // (gather batch U, resident CTAs per SM) of a variant code for element size elem.
 void variant_params(int code, int elem, int *V, int *U, int *MB);
 
+// Steps of a chain operator from a list of every row's flips (pf_chain_step.cu),
+// for callers that take many: its bytes (0: not offered), its making, and the
+// step, as launch_step on contiguous rows with Q among the flags.
+size_t chain_list_bytes(const pf_op *op);
+void build_chain_list(pf_op *op, cudaStream_t st, void *list);
+template <typename T>
+void launch_chain_listed(pf_op *op, cudaStream_t st, const void *list, int s, const T *q, const T *p, const T *x, T *out,
+                         double cx, double alpha, double beta, double inva, double shift, int flags, double *dots);
+
 // RI <-> column-major conversion, optional precision change.
 template <typename TS, typename TD>
 void launch_cm_to_ri(cudaStream_t st, int64_t D, int s, const TS *src, int64_t ld, TD *dst);

@@ -25,7 +25,7 @@
 //     of (outer bit, grain bit) with value g0 c_j / 4, plus the dense grain
 //     block on the low L_grain bits (held in shared memory).
 #include "pf_internal.h"
-#include "pf_rows.cuh"
+#include "pf_step.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -33,24 +33,6 @@
 #include <mutex>
 
 namespace pf {
-
-template <typename T>
-struct StepArgs {
-    uint32_t D;
-    int s;          // columns processed per row
-    int ld;         // row stride of the blocks (>= s: a column slab of a wider RI block)
-    int stream;     // 1: x, p and out move with evict-first hints (slab passes)
-    int G;          // column groups per row = s / V
-    uint32_t items; // D * G
-    const T *q;
-    const T *p;     // may alias out (in-place update)
-    const T *x;
-    T *out;
-    T cx, alpha, beta, inva, boa;
-    double *partials;
-    unsigned int *counter;
-    double *dots;
-};
 
 template <class Desc>
 struct DescTraits;
@@ -66,39 +48,6 @@ template <typename T>
 struct DescTraits<CsrDesc<T>> {
     static constexpr int kind = OP_CSR;
 };
-
-constexpr int kThreads = 256;
-
-// Deterministic "last block reduces" epilogue: every block writes its
-// per-column partials, the block that finishes last sums them in block order.
-// The partials are read through L2 (__ldcg: other blocks wrote them before
-// the counter told this block it is last) in unrolled runs, so a run's loads
-// are in flight together while the sum keeps block order.
-__device__ void finish_reduction(int nvals, const double *blockvals, double *partials,
-                                 unsigned int *counter, double *out) {
-    __shared__ bool last;
-    for (int c = threadIdx.x; c < nvals; c += blockDim.x)
-        partials[(size_t)blockIdx.x * nvals + c] = blockvals[c];
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int t = atomicAdd(counter, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last) {
-        __threadfence();
-        const unsigned int nb = gridDim.x;
-        for (int c = threadIdx.x; c < nvals; c += blockDim.x) {
-            double acc = 0.0;
-            const double *col = partials + c;
-#pragma unroll 8
-            for (unsigned int b = 0; b < nb; ++b) acc += __ldcg(col + (size_t)b * nvals);
-            out[c] = acc;
-        }
-        if (threadIdx.x == 0) *counter = 0u;
-    }
-}
 
 // UB > 0 / MB > 0: a tuned variant's gather batch and resident-CTA target
 // (register cap); 0 keeps the defaults of Batch / MinBlocks.  RK = 1 (chain
@@ -196,51 +145,7 @@ __global__ void __launch_bounds__(kThreads, MB > 0 ? MB : MinBlocks<T, V>::value
         }
     }
 
-    if constexpr (DOTS) {
-        // Every item of a thread has column group threadIdx.x % G (G divides the
-        // grid stride; checked on the host).  Lanes of one group are first
-        // summed with warp shuffles, then per warp in shared memory.
-        const int Gi = a.G;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if (Gi < 32) {
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-                for (int o = 16; o >= Gi; o >>= 1) {
-                    dd1[v] += __shfl_xor_sync(0xffffffffu, dd1[v], o);
-                    dd2[v] += __shfl_xor_sync(0xffffffffu, dd2[v], o);
-                }
-        }
-        const int lanes = Gi < 32 ? Gi : 32;
-        __syncthreads();
-        double *red = reinterpret_cast<double *>(smem_raw);  // [8 warps][lanes][2V]
-        if (lane < lanes)
-            for (int v = 0; v < V; ++v) {
-                red[(warp * lanes + lane) * 2 * V + v] = dd1[v];
-                red[(warp * lanes + lane) * 2 * V + V + v] = dd2[v];
-            }
-        __syncthreads();
-        double *bv = red + (kThreads / 32) * lanes * 2 * V;  // [2 s]
-        for (int c = threadIdx.x; c < a.s; c += blockDim.x) {
-            const int g = c / V, v = c - g * V;
-            double s1 = 0.0, s2 = 0.0;
-            if (Gi < 32) {
-                for (int w = 0; w < kThreads / 32; ++w) {
-                    s1 += red[(w * lanes + g) * 2 * V + v];
-                    s2 += red[(w * lanes + g) * 2 * V + V + v];
-                }
-            } else {
-                for (int t = g; t < kThreads; t += Gi) {
-                    const int w = t >> 5, l = t & 31;
-                    s1 += red[(w * lanes + l) * 2 * V + v];
-                    s2 += red[(w * lanes + l) * 2 * V + V + v];
-                }
-            }
-            bv[c] = s1;
-            bv[a.s + c] = s2;
-        }
-        __syncthreads();
-        finish_reduction(2 * a.s, bv, a.partials, a.counter, a.dots);
-    }
+    if constexpr (DOTS) step_dots<V>(dd1, dd2, a.G, a.s, smem_raw, a.partials, a.counter, a.dots);
 }
 
 // ------------------------------------------------ warp-cooperative chain step
@@ -601,24 +506,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// Launches a step kernel on st, with programmatic dependent launch when the
-// handle allows it (the kernels wait for their predecessor themselves).
-template <typename... KArgs, typename... Args>
-static void launch_step_kernel(pf_handle *h, void (*kern)(KArgs...), int grid, int smem, cudaStream_t st,
-                               Args &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = h->overlap ? 1 : 0;
-    PF_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
-}
-
 static thread_local int64_t t_launches = 0;
 void count_launches(int64_t n) { t_launches += n; }
 int64_t thread_launches() { return t_launches; }
@@ -645,7 +532,7 @@ void ensure_reduction(pf_handle *h, size_t n) {
 
 // Resident CTAs per SM of a kernel instance (occupancy calculator, cached per
 // host thread so concurrent solves do not contend on a lock every launch).
-static int blocks_per_sm(const void *kern, int smem) {
+int step_blocks_per_sm(const void *kern, int smem) {
     thread_local std::map<std::pair<const void *, int>, int> cache;
     auto key = std::make_pair(kern, smem);
     auto it = cache.find(key);
@@ -661,7 +548,7 @@ static int blocks_per_sm(const void *kern, int smem) {
 // refused (PF_ERR_UNSUPPORTED) instead of timed.
 thread_local bool t_refuse_spilling = false;
 
-static bool spills(const void *kern) {
+bool step_spills(const void *kern) {
     thread_local std::map<const void *, bool> cache;
     auto it = cache.find(kern);
     if (it != cache.end()) return it->second;
@@ -673,12 +560,12 @@ static bool spills(const void *kern) {
 template <typename T, int V, class Desc, int FLAGS, int UB = 0, int MB = 0, int RK = 0>
 static void launch_one(pf_op *op, cudaStream_t st, const Desc &d, StepArgs<T> a, int smem) {
     auto kern = k_step<T, V, Desc, FLAGS, UB, MB, RK>;
-    if (t_refuse_spilling && spills((const void *)kern))
+    if (t_refuse_spilling && step_spills((const void *)kern))
         throw Error(PF_ERR_UNSUPPORTED, "step-kernel variant spills registers");
     if (smem > 48 * 1024) PF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     // one item per thread when the whole block fits on the device at once,
     // otherwise a persistent grid of every resident CTA
-    const int grid = grid_for(op->h, a.items, kThreads, blocks_per_sm((const void *)kern, smem));
+    const int grid = grid_for(op->h, a.items, kThreads, step_blocks_per_sm((const void *)kern, smem));
     if constexpr ((FLAGS & StepFlags::DOTS) != 0) {
         ensure_reduction(op->h, (size_t)grid * 2 * a.s);
         a.partials = op->h->red_partials;
@@ -770,7 +657,7 @@ static void launch_qsun_async_one(pf_op *op, cudaStream_t st, const QSunDesc<T> 
     auto kern = k_step_qsun_async<T, V, FLAGS>;
     const int smem = qsun_async_smem(d, V);
     PF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const int grid = grid_for(op->h, a.items, kThreads, blocks_per_sm((const void *)kern, smem));
+    const int grid = grid_for(op->h, a.items, kThreads, step_blocks_per_sm((const void *)kern, smem));
     launch_step_kernel(op->h, kern, grid, smem, st, d, a);
     PF_CUDA(cudaGetLastError());
     count_launches(1);
@@ -842,14 +729,14 @@ const float *qsun_tabs<float>(const pf_op *op) { return static_cast<const float 
 template <typename T, int V, int FLAGS, int IPT>
 static void launch_qsun_tile_one(pf_op *op, cudaStream_t st, const QSunDesc<T> &d, const StepArgs<T> &a, int tbits) {
     auto kern = k_step_qsun_tile<T, V, FLAGS, IPT>;
-    if (t_refuse_spilling && spills((const void *)kern))
+    if (t_refuse_spilling && step_spills((const void *)kern))
         throw Error(PF_ERR_UNSUPPORTED, "step-kernel variant spills registers");
     const int smem = qsun_tile_offset<T>() + (int)(((int64_t)1 << tbits) * a.s * (int64_t)sizeof(T));
     if (smem > 48 * 1024) PF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     // one CTA per tile (the scheduler balances them) up to 8 waves, then a
     // persistent loop over the tiles
     const int64_t ntiles = (int64_t)a.D >> tbits;
-    const int64_t cap = (int64_t)op->h->num_sms * blocks_per_sm((const void *)kern, smem) * 8;
+    const int64_t cap = (int64_t)op->h->num_sms * step_blocks_per_sm((const void *)kern, smem) * 8;
     const int grid = (int)std::max<int64_t>(1, std::min(ntiles, cap));
     launch_step_kernel(op->h, kern, grid, smem, st, d, a, qsun_tabs<T>(op), tbits);
     PF_CUDA(cudaGetLastError());
@@ -886,8 +773,7 @@ static bool launch_qsun_tile(pf_op *op, cudaStream_t st, const QSunDesc<T> &d, c
 template <typename T, int V>
 static void dispatch_op(pf_op *op, cudaStream_t st, const StepArgs<T> &a, int flags, int profile) {
     int smem = 0;
-    const int lanes = a.G < 32 ? a.G : 32;
-    const int dots_smem = (kThreads / 32) * lanes * 2 * V * 8 + 2 * a.s * 8;
+    const int dots_smem = step_dots_smem(a.G, V, a.s);
     if (op->kind == OP_CHAIN) {
         const ChainDesc<T> &d = chain_of<T>(op);
         if ((flags & StepFlags::Q) && !d.full) smem = rank_table_entries(d.nchunks) * 4;
@@ -921,7 +807,7 @@ static void launch_coop_one(pf_op *op, cudaStream_t st, const ChainDesc<T> &d, c
     int smem = PF_MAX_BONDS * 4;
     if ((FLAGS & StepFlags::Q) && !d.full) smem += rank_table_entries(d.nchunks) * 4;
     if (smem > 48 * 1024) PF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const int grid = grid_for(op->h, (int64_t)a.D * S, kThreads, blocks_per_sm((const void *)kern, smem));
+    const int grid = grid_for(op->h, (int64_t)a.D * S, kThreads, step_blocks_per_sm((const void *)kern, smem));
     launch_step_kernel(op->h, kern, grid, smem, st, d, a);
     PF_CUDA(cudaGetLastError());
     count_launches(1);
@@ -1134,7 +1020,7 @@ __global__ void __launch_bounds__(kThreads) k_coldots(uint32_t D, int s, uint32_
         bv[c] = acc;
     }
     __syncthreads();
-    finish_reduction(s, bv, partials, counter, out);
+    finish_reduction(s, bv, partials, counter, out, bv + s);
 }
 
 __global__ void __launch_bounds__(kThreads) k_colresid(uint32_t D, int s, uint32_t rows_per_block,
@@ -1155,7 +1041,7 @@ __global__ void __launch_bounds__(kThreads) k_colresid(uint32_t D, int s, uint32
         bv[c] = acc;
     }
     __syncthreads();
-    finish_reduction(s, bv, partials, counter, out);
+    finish_reduction(s, bv, partials, counter, out, bv + s);
 }
 
 // For narrow blocks (s < 64) the per-column loops above leave most threads
@@ -1184,7 +1070,7 @@ __global__ void __launch_bounds__(kThreads) k_coldots_narrow(uint32_t D, int s, 
         bv[c] = a;
     }
     __syncthreads();
-    finish_reduction(s, bv, partials, counter, out);
+    finish_reduction(s, bv, partials, counter, out, bv + s);
 }
 
 template <typename T>
@@ -1192,7 +1078,7 @@ void launch_coldots(pf_handle *h, cudaStream_t st, int64_t D, int s, const T *A,
     if (s < 64) {
         int grid = grid_for(h, D * s, kThreads, 2);
         ensure_reduction(h, (size_t)grid * s);
-        size_t smem = (kThreads + s) * sizeof(double);
+        size_t smem = (2 * kThreads + s) * sizeof(double);
         k_coldots_narrow<T><<<grid, kThreads, smem, st>>>((uint32_t)D, s, A, B, h->red_partials,
                                                           h->red_counter, out);
         count_launches(1);
@@ -1204,7 +1090,7 @@ void launch_coldots(pf_handle *h, cudaStream_t st, int64_t D, int s, const T *A,
             grid = (int)((D + rpb - 1) / rpb);
         }
         ensure_reduction(h, (size_t)grid * s);
-        size_t smem = s * sizeof(double);
+        size_t smem = (s + kThreads) * sizeof(double);
         if (smem > 48 * 1024) PF_CUDA(cudaFuncSetAttribute(k_coldots<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_coldots<T><<<grid, kThreads, smem, st>>>((uint32_t)D, s, rpb, A, B, h->red_partials,
                                                    h->red_counter, out);
@@ -1224,7 +1110,7 @@ void launch_colresid(pf_handle *h, cudaStream_t st, int64_t D, int s, const doub
         grid = (int)((D + rpb - 1) / rpb);
     }
     ensure_reduction(h, (size_t)grid * s);
-    size_t smem = s * sizeof(double);
+    size_t smem = (s + kThreads) * sizeof(double);
     if (smem > 48 * 1024) PF_CUDA(cudaFuncSetAttribute(k_colresid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_colresid<<<grid, kThreads, smem, st>>>((uint32_t)D, s, rpb, HA, A, e, h->red_partials, h->red_counter, out);
     count_launches(1);

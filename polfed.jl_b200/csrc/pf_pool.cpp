@@ -100,6 +100,7 @@ double solve_footprint(const pf_op *op, const pf_params *p, int s, int nev) {
     bytes += 2.0 * D * 64 * w;                                        // KPM probe blocks
     bytes += 2.0 * 8.0 * D * nev;                                     // Ritz vectors and H psi
     bytes += 3.0 * 8.0 * maxdim * maxdim + (64 << 20);                // projected matrix, its eigenvectors, slack
+    bytes += (double)chain_list_bytes(op);                            // a chain's flip list
     return bytes;
 }
 

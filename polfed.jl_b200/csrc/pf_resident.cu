@@ -817,16 +817,14 @@ static int res_resident(const ResPlan &p) {
 }
 
 // A filter step of ncol columns by the step kernels, in us: what the autotuned
-// kernels measured over D = 2^11 .. 2^17 (a launch floor, then the gathered
-// values); chains run at a different rate where the warp-cooperative step is
-// offered.  KPM steps (fused dots) are about twice that.
+// kernels, or a chain's listed ones, measured over D = 2^11 .. 2^17 (a launch
+// floor, then the gathered values).  KPM steps (fused dots) are about twice that.
 static double step_us(const pf_op *op, int ncol, int elem, bool kpm) {
     const double D = (double)op->dim, w = elem == 8 ? 1.0 : 0.7;
     double us;
     if (op->kind == OP_QSUN) us = 2.8 + D * ncol * (op->L_loc + (1 << op->L_grain)) * 0.42e-6 * w;
     else if (op->kind == OP_CSR) us = 2.8 + D * ncol * list_terms(op) * 1.15e-6 * w;
-    else if (coop_eligible(op, ncol, 0)) us = 2.6 + D * ncol * list_terms(op) * 2.0e-6 * w;
-    else us = 6.0 + D * ncol * list_terms(op) * 4.0e-6 * w;
+    else us = 3.0 + D * ncol * list_terms(op) * 0.9e-6 * (elem == 8 ? 1.0 : 0.5);
     return kpm ? 2 * us : us;
 }
 

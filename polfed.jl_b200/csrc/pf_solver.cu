@@ -124,17 +124,50 @@ struct StageClock {
 
 static void sync(pf_handle *h) { PF_CUDA(cudaStreamSynchronize(h->stream)); }
 
+// ------------------------------------------------------------ listed chains
+// A chain's flip list for the steps of one call (chain_list_bytes), held while
+// it lives; empty for other operators and where it would take more than a
+// sixteenth of the device's memory (or does not fit): the steps then rank their
+// flips themselves.
+static size_t device_bytes(int device) {
+    thread_local std::map<int, size_t> known;
+    auto it = known.find(device);
+    if (it != known.end()) return it->second;
+    size_t free_b = 0, total_b = 0;
+    PF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    return known[device] = total_b;
+}
+struct ChainList {
+    DevArray<unsigned char> mem;
+    const void *get() const { return mem.p; }
+    void make(pf_op *op, cudaStream_t st) {
+        const size_t bytes = chain_list_bytes(op);
+        if (bytes == 0 || mem.p || bytes > device_bytes(op->h->device) / 16) return;
+        try {
+            mem.alloc(bytes);
+        } catch (const Error &e) {
+            if (e.code != PF_ERR_NOMEM) throw;
+            cudaGetLastError();
+            return;
+        }
+        build_chain_list(op, st, mem.p);
+    }
+};
+// Steps from which a call makes its own list: making it takes about as long as
+// one step with it, and a step with it two thirds of one without.
+constexpr int kListSteps = 8;
+
 // ------------------------------------------------------------ the filter
 // Whether an s-column filter runs whole on chip: it fits and is estimated
 // faster than the step kernels, and the caller asked for neither column slabs
 // nor a step variant of their own.
+static bool pinned_step(pf_op *op, int s, int elem) {
+    std::lock_guard<std::mutex> lock(op->tune_mu);
+    return op->pinned_width.count(std::make_pair(elem, s)) > 0;
+}
 template <typename T>
 static bool resident_filter_plan(pf_op *op, int s, ResPlan *plan) {
-    {
-        std::lock_guard<std::mutex> lock(op->tune_mu);
-        if (op->pinned_width.count(std::make_pair((int)sizeof(T), s))) return false;
-    }
-    return op->slab_cols <= 0 && resident_plan<T>(op, s, false, plan);
+    return op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T)) && resident_plan<T>(op, s, false, plan);
 }
 
 // Y = sum_k c_k T_k(Htilde) X on RI blocks (ClenshawAlgorithm.jl:12-29).
@@ -151,14 +184,17 @@ struct Filter {
     bool resident;
     DevArray<unsigned char> work;
     DevArray<double> dc;
+    ChainList own_list;   // of a chain, unless the caller has one
+    const void *list;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 
     // io = false: only the two work blocks (the filter engine reads and
     // writes the caller's blocks directly)
-    Filter(pf_op *op_, int s_, const std::vector<double> &coeffs, double a_, double b_, bool io = true)
+    Filter(pf_op *op_, int s_, const std::vector<double> &coeffs, double a_, double b_, bool io = true,
+           const void *list_ = nullptr)
         : op(op_), s(s_), K((int)coeffs.size() - 1), c(coeffs), a(a_), b(b_),
-          resident(io && resident_filter_plan<T>(op_, s_, &plan)) {
+          resident(io && resident_filter_plan<T>(op_, s_, &plan)), list(nullptr) {
         const size_t n = (size_t)op->dim * s;
         if (resident) {
             dc.alloc(c.size());
@@ -173,6 +209,13 @@ struct Filter {
         }
         if (K >= 1) A.alloc(n);
         if (K >= 2) B.alloc(n);
+        if (io && op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T))) {
+            list = list_;
+            if (!list && K >= kListSteps) {
+                own_list.make(op, op->h->stream);
+                list = own_list.get();
+            }
+        }
     }
     // the fixed input and output blocks (a resident filter allocates them on first use)
     T *x() {
@@ -206,6 +249,10 @@ struct Filter {
     void step(cudaStream_t st, const T *q, const T *p, T *out, double ck, double alpha, double beta, int flags) {
         const int w = slab_cols();
         const int64_t D = op->dim;
+        if (list && (flags & StepFlags::Q)) {
+            launch_chain_listed<T>(op, st, list, s, q, p, X.p, out, ck, alpha, beta, 1.0 / a, b, flags, nullptr);
+            return;
+        }
         for (int c0 = 0; c0 < s; c0 += w)
             launch_step<T>(op, st, D, w, q ? q + c0 : nullptr, p ? p + c0 : nullptr, X.p + c0, out + c0, ck, alpha, beta,
                            1.0 / a, b, flags, nullptr, w == s ? 0 : s, w == s ? 0 : 1);
@@ -266,7 +313,8 @@ struct Filter {
 // power-of-two column blocks of at most 64.
 template <typename T>
 static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int R, const T *probes_cm,
-                                       int64_t ldp, int kind, uint64_t seed, int64_t *block_matvecs) {
+                                       int64_t ldp, int kind, uint64_t seed, int64_t *block_matvecs,
+                                       const void *list = nullptr) {
     pf_handle *h = op->h;
     const int64_t D = op->dim;
     cudaStream_t st = h->stream;
@@ -303,6 +351,15 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
     DevArray<T> v0((size_t)D * RB), v1((size_t)D * RB);
     DevArray<double> dots((size_t)std::max(M, 1) * 2 * RB), n0(RB), scl(RB);
     std::vector<double> hd((size_t)std::max(M, 1) * 2 * RB), h0(RB), hs(RB);
+    ChainList own_list;
+    if (!list && (int64_t)M * ((R + 63) / 64) >= kListSteps) {
+        own_list.make(op, st);
+        list = own_list.get();
+    }
+    auto step = [&](int nb, const T *q, const T *p, T *out, double alpha, double beta, int flags, double *dst) {
+        if (list) launch_chain_listed<T>(op, st, list, nb, q, p, nullptr, out, 0, alpha, beta, 1.0 / a, b, flags, dst);
+        else launch_step<T>(op, st, D, nb, q, p, nullptr, out, 0, alpha, beta, 1.0 / a, b, flags, dst);
+    };
     int64_t mv = 0;
     int c0 = 0;
     while (c0 < R) {
@@ -322,11 +379,10 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
         }
         launch_coldots<T>(h, st, D, nb, prev, prev, n0.p);
         if (M >= 1) {
-            launch_step<T>(op, st, D, nb, prev, nullptr, nullptr, cur, 0, 1.0, 0, 1.0 / a, b,
-                           StepFlags::Q | StepFlags::DOTS, dots.p);
+            step(nb, prev, nullptr, cur, 1.0, 0, StepFlags::Q | StepFlags::DOTS, dots.p);
             for (int n = 1; n < M; ++n) {
-                launch_step<T>(op, st, D, nb, cur, prev, nullptr, prev, 0, 2.0, -1.0, 1.0 / a, b,
-                               StepFlags::Q | StepFlags::P | StepFlags::DOTS, dots.p + (size_t)n * 2 * nb);
+                step(nb, cur, prev, prev, 2.0, -1.0, StepFlags::Q | StepFlags::P | StepFlags::DOTS,
+                     dots.p + (size_t)n * 2 * nb);
                 std::swap(prev, cur);
             }
         }
@@ -1206,7 +1262,7 @@ static void cholqr2_block(pf_handle *h, double *W, int64_t D, int m) {
 // Returns the number of passes run.
 static int refine_fp64(pf_op *op, const std::vector<double> &coeffs, double a, double b, int nev, double eigentol,
                        int max_passes, DevArray<double> &Psi, int m, std::vector<double> &vals,
-                       std::vector<double> &resid) {
+                       std::vector<double> &resid, const void *list) {
     pf_handle *h = op->h;
     cudaStream_t st = h->stream;
     const int64_t D = op->dim;
@@ -1231,7 +1287,7 @@ static int refine_fp64(pf_op *op, const std::vector<double> &coeffs, double a, d
         for (int c0 = 0; c0 < m; c0 += wmax) {
             const int wc = std::min(wmax, m - c0);
             auto &f = filters[wc];
-            if (!f) f.reset(new Filter<double>(op, wc, coeffs, a, b));
+            if (!f) f.reset(new Filter<double>(op, wc, coeffs, a, b, true, list));
             if (f->resident) {
                 f->run_resident(st, Psi.p + c0, m, 1, W.p + c0, m, 1);
                 continue;
@@ -1307,8 +1363,14 @@ static pf_handle *aux_handle(pf_handle *h) {
 }
 
 static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, double tol, double eigentol, double *Emin,
-                                double *Emax, int *qr_restarts = nullptr, bool host_qr = false) {
+                                double *Emax, int *qr_restarts = nullptr, bool host_qr = false,
+                                const void *list = nullptr) {
     const int64_t D = op->dim;
+    ChainList own_list;
+    if (!list) {
+        own_list.make(op, op->h->stream);
+        list = own_list.get();
+    }
     // The :SR probe runs here and the :LR probe at the same time on the
     // auxiliary handle (its own stream, cuBLAS and cuSOLVER): both only read
     // v0, so each gives exactly what it gives alone.
@@ -1320,8 +1382,12 @@ static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, dou
     PF_CUDA(cudaStreamWaitEvent(ah->stream, ready, 0));
     auto probe = [&](pf_op *o, int which, double *out) -> int {
         BlockMap happly = [&](const double *X, double *Y) {
-            launch_step<double>(o, o->h->stream, D, 1, X, nullptr, nullptr, Y, 0, 1.0, 0, 1.0, 0.0, StepFlags::Q,
-                                nullptr);
+            if (list)
+                launch_chain_listed<double>(o, o->h->stream, list, 1, X, nullptr, nullptr, Y, 0, 1.0, 0, 1.0, 0.0,
+                                            StepFlags::Q, nullptr);
+            else
+                launch_step<double>(o, o->h->stream, D, 1, X, nullptr, nullptr, Y, 0, 1.0, 0, 1.0, 0.0, StepFlags::Q,
+                                    nullptr);
         };
         LanczosOut lo;
         lanczos(o, 1, 1, maxdim, tol, eigentol, which, 1, v0_dev, happly, lo, nullptr, -1, host_qr);
@@ -1353,6 +1419,7 @@ static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, dou
     }
     t.join();
     cudaEventDestroy(ready);
+    if (aux_err) cudaStreamSynchronize(ah->stream);   // what it still runs reads the list
     count_launches(aux_launches);
     if (err) std::rethrow_exception(err);
     if (aux_err) std::rethrow_exception(aux_err);
@@ -1537,6 +1604,12 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     PF_CUDA(cudaMemcpyAsync(xcm.p, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     launch_cm_to_ri<double, double>(st, D, s, xcm.p, D, xri.p);
 
+    // a chain's flips are listed once for the whole solve (its probes, its
+    // moments and its filter), unless the solve itself is near the device's memory
+    ChainList chain_list;
+    if (solve_footprint(op, P, s, nev) < 0.85 * (double)device_bytes(h->device)) chain_list.make(op, st);
+    const void *list = chain_list.get();
+
     // mapping plan (Plan.jl:128-191)
     double Emin = P->Emin, Emax = P->Emax;
     {
@@ -1545,7 +1618,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
             double lo = 0, hi = 0;
             // v0 = x0[:, 1] (column 0 of the column-major copy)
             extrema_from_device(op, xcm.p, P->extrema_maxdim > 0 ? P->extrema_maxdim : 1000, 1e-14, 1e-8, &lo, &hi,
-                                &R.qr_restarts, P->host_qr != 0);
+                                &R.qr_restarts, P->host_qr != 0, list);
             if (!P->has_Emin) Emin = lo;
             if (!P->has_Emax) Emax = hi;
         }
@@ -1588,14 +1661,16 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
             PF_CUDA(cudaMemcpyAsync(pr64.p, P->probes, pr64.n * sizeof(double), cudaMemcpyHostToDevice, st));
         }
         if (P->precision == PF_PREC_FP64) {
-            mu = kpm_moments<double>(op, a, b, P->dos_N, P->dos_R, pr64.p, D, P->probe_kind, P->seed, &R.kpm_block_matvecs);
+            mu = kpm_moments<double>(op, a, b, P->dos_N, P->dos_R, pr64.p, D, P->probe_kind, P->seed, &R.kpm_block_matvecs,
+                                     list);
         } else {
             if (P->probes) {
                 pr32.alloc((size_t)D * P->dos_R);
                 // FP64 host probes -> FP32 device copy (column-major kept)
                 launch_ri_to_cm<double, float>(st, (int64_t)P->dos_R * D, 1, pr64.p, pr32.p, (int64_t)P->dos_R * D);
             }
-            mu = kpm_moments<float>(op, a, b, P->dos_N, P->dos_R, pr32.p, D, P->probe_kind, P->seed, &R.kpm_block_matvecs);
+            mu = kpm_moments<float>(op, a, b, P->dos_N, P->dos_R, pr32.p, D, P->probe_kind, P->seed, &R.kpm_block_matvecs,
+                                    list);
         }
         R.stage_seconds[7] = std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count();
     }
@@ -1622,7 +1697,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     ResPlan onchip;
     const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, &onchip)
                                                  : resident_filter_plan<float>(op, s, &onchip));
-    if (P->autotune && steps) {
+    if (P->autotune && steps && (eng || !list || op->slab_cols > 0)) {
         bool have;
         {
             std::lock_guard<std::mutex> lock(op->tune_mu);
@@ -1632,7 +1707,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     }
     const int ew = engine_width(op, s, fdtype == PF_F64 ? 8 : 4);
     if (P->precision == PF_PREC_FP64) {
-        Filter<double> filt(op, s, coeffs, a, b, eng == nullptr);
+        Filter<double> filt(op, s, coeffs, a, b, eng == nullptr, list);
         BlockMap fmap = [&](const double *X, double *Y) {
             if (eng) {
                 engine_filter(eng, op, st, 8, s, ew, coeffs, a, b, (void *)X, Y, filt.A.p, filt.B.p);
@@ -1654,7 +1729,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
         // last target is the filter ratio P(lambda_{2 nev}) / P(lambda_{nev})
         const int guard = std::max(s, nev);
         {
-            Filter<float> filt(op, s, coeffs, a, b, eng == nullptr);
+            Filter<float> filt(op, s, coeffs, a, b, eng == nullptr, list);
             BlockMap fmap = [&](const double *X, double *Y) {
                 launch_ri_to_cm<double, float>(st, (int64_t)D * s, 1, X, filt.x(), (int64_t)D * s);
                 if (eng) engine_filter(eng, op, st, 4, s, ew, coeffs, a, b, filt.x(), filt.y(), filt.A.p, filt.B.p);
@@ -1671,7 +1746,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
             int before = 0;
             while (before < nev && before < m && out.resid[before] < P->eigentol) ++before;
             std::vector<double> vals_f(out.vals), resid(out.resid);
-            refine_fp64(op, coeffs, a, b, nev, P->eigentol, P->refine, out.vecs, m, vals_f, resid);
+            refine_fp64(op, coeffs, a, b, nev, P->eigentol, P->refine, out.vecs, m, vals_f, resid, list);
             int ec = 0;
             double maxe = 0.0;
             bool counting = true;
