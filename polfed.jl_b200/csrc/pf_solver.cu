@@ -1567,6 +1567,78 @@ static void prepare_initial_state(std::vector<double> &x, int64_t D, int s) {
         for (int c = 0; c < s; ++c) x[r + c * D] = A[r * s + c];
 }
 
+// The same on the device for an RI block X of at most kBlkMaxS columns, with
+// the Gram and solve passes of the Lanczos iteration (pf_blocks.cu) and CholQR2
+// in place of the Householder factors: the same column space, each column up
+// to its sign.  On the host the Gram matrix and the factorisation of the
+// 65536 x 8 start took 40 ms, an eighth of the solve.  Returns false, with X as
+// it was, where the host form has to decide: entries that are not finite (or
+// whose squares overflow), a zero column, a numerically dependent block.
+static bool prepare_initial_state_device(pf_op *op, int s, double *X) {
+    pf_handle *h = op->h;
+    cudaStream_t st = h->stream;
+    const int64_t D = op->dim;
+    if (s > kBlkMaxS) return false;
+    const size_t ss = (size_t)s * s, n = (size_t)D * s;
+    DevArray<double> W(n), small(2 * ss), part(blk_partial_doubles(D, s));
+    DevArray<unsigned> count(blk_counters());
+    PF_CUDA(cudaMemsetAsync(count.p, 0, blk_counters() * sizeof(unsigned), st));
+    double *pin = pinned_scratch(h, ss);
+    auto pass = [&](double *block, int flags) {
+        BlkPass p;
+        p.D = D;
+        p.s = s;
+        p.W = block;
+        p.flags = flags;
+        p.Rs = small.p + ss;
+        p.partial = part.p;
+        p.counter = count.p;
+        p.G = small.p;
+        blk_pass(st, p);
+    };
+    auto gram = [&](std::vector<double> &G) {
+        PF_CUDA(cudaMemcpyAsync(pin, small.p, ss * sizeof(double), cudaMemcpyDeviceToHost, st));
+        sync(h);
+        G.assign(pin, pin + ss);
+    };
+    auto upload = [&](const std::vector<double> &R) {
+        std::memcpy(pin, R.data(), ss * sizeof(double));
+        PF_CUDA(cudaMemcpyAsync(small.p + ss, pin, ss * sizeof(double), cudaMemcpyHostToDevice, st));
+    };
+    std::vector<double> G, R;
+    pass(X, BLK_GRAM);
+    gram(G);
+    double dn = 0.0, gn = 0.0;
+    for (int i = 0; i < s; ++i)
+        for (int j = 0; j < s; ++j) {
+            const double e = G[i + j * s] - (i == j ? 1.0 : 0.0);
+            dn += e * e;
+            gn += G[i + j * s] * G[i + j * s];
+        }
+    if (!std::isfinite(gn)) return false;
+    const double tol = 1e-10;
+    if (s == 1) {
+        const double nrm = std::sqrt(G[0]);
+        if (nrm == 0.0) return false;
+        if (std::fabs(nrm - 1.0) <= std::max(tol, tol * std::max(nrm, 1.0))) return true;
+        R.assign(1, nrm);
+        upload(R);
+        pass(X, BLK_SOLVE);
+        return true;
+    }
+    if (std::sqrt(dn) <= std::max(tol, tol * std::max(std::sqrt(gn), std::sqrt((double)s)))) return true;
+    if (!host_cholesky(G, s, R)) return false;
+    upload(R);
+    PF_CUDA(cudaMemcpyAsync(W.p, X, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    pass(W.p, BLK_SOLVE | BLK_GRAM);
+    gram(G);
+    if (!host_cholesky(G, s, R)) return false;
+    upload(R);
+    pass(W.p, BLK_SOLVE);
+    PF_CUDA(cudaMemcpyAsync(X, W.p, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    return true;
+}
+
 void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int x0_mem, double *vals, double *vecs,
            int vecs_mem, pf_report *rep, int *nconv) {
     PF_CHECK(op && P && x0 && vals && nconv, PF_ERR_INVALID, "null argument");
@@ -1591,18 +1663,22 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     PF_CUDA(cudaEventRecord(t_begin, st));
     auto t_wall0 = std::chrono::steady_clock::now();
 
-    // x0 -> host column-major, validate / orthonormalise, -> device RI
-    std::vector<double> hx((size_t)D * s);
-    if (x0_mem == PF_MEM_DEVICE)
-    {
-        PF_CUDA(cudaMemcpyAsync(hx.data(), x0, hx.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    // x0 -> device RI, validated and orthonormalised there, else on the host
+    DevArray<double> xcm((size_t)D * s), xri((size_t)D * s);
+    PF_CUDA(cudaMemcpyAsync(xcm.p, x0, (size_t)D * s * sizeof(double),
+                            x0_mem == PF_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+    launch_cm_to_ri<double, double>(st, D, s, xcm.p, D, xri.p);
+    if (prepare_initial_state_device(op, s, xri.p)) {
+        launch_ri_to_cm<double, double>(st, D, s, xri.p, xcm.p, D);
+    } else {
+        std::vector<double> hx((size_t)D * s);
+        PF_CUDA(cudaMemcpyAsync(hx.data(), xcm.p, hx.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        sync(h);
+        prepare_initial_state(hx, D, s);
+        PF_CUDA(cudaMemcpyAsync(xcm.p, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        launch_cm_to_ri<double, double>(st, D, s, xcm.p, D, xri.p);
         sync(h);
     }
-    else std::memcpy(hx.data(), x0, hx.size() * sizeof(double));
-    prepare_initial_state(hx, D, s);
-    DevArray<double> xcm((size_t)D * s), xri((size_t)D * s);
-    PF_CUDA(cudaMemcpyAsync(xcm.p, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    launch_cm_to_ri<double, double>(st, D, s, xcm.p, D, xri.p);
 
     // a chain's flips are listed once for the whole solve (its probes, its
     // moments and its filter), unless the solve itself is near the device's memory
