@@ -14,7 +14,7 @@ std::vector<double> raw_coefficients(double target, int K);
 class Dos {
   public:
     Dos(const std::vector<double> &mu, int N, int kernel);
-    double operator()(double x) const;
+    void eval(const double *x, double *y, int n) const;   // rho at n points
 
   private:
     int N_;
@@ -22,8 +22,9 @@ class Dos {
 };
 
 double bisection(const std::function<int(double)> &f, double x1, double x2, double tol, int max_iter);
-double quadgk(const std::function<double(double)> &f, double a, double b, double atol, double rtol,
-              long maxevals);
+// f: its values at n points
+double quadgk(const std::function<void(const double *, double *, int)> &f, double a, double b, double atol,
+              double rtol, long maxevals);
 double analytical_order(double lam, double delta);
 
 // TransformPlan of Plan.jl:32-44 in rescaled units.
