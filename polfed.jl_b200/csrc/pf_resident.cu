@@ -54,6 +54,10 @@ struct ResArgs {
     // others), and the exchange inside the chunk
     uint32_t flip[PF_MAX_LOC];
     uint8_t inner[PF_MAX_LOC];
+    // Quantum Sun filters of more columns than clusters fit the device at once:
+    // `slots` > 0 launches of that many columns, each for `steps` steps
+    int slot, slots, steps;
+    T *state;            // [columns][2][D]: a column's vectors between its slots
     T *xch;              // exchange blocks [2][columns][D], or null: CTAs read each other's shared memory
 };
 
@@ -219,7 +223,16 @@ __global__ void __launch_bounds__(ResQSun<T, LG>::threads)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int clog = a.clog, C = 1 << clog;
     const uint32_t rank = clog ? cluster_rank() : 0u;
-    const int col = blockIdx.x >> clog;
+    int col = blockIdx.x >> clog;
+    int n0 = 0, n1 = a.K;                // steps of this launch
+    if (!KPM && a.slots > 0) {
+        col = (col + a.slot) % a.ncol;
+        int before = 0;                  // earlier launches with this column
+        for (int j = 0; j < a.slot; ++j) before += (col - j + a.ncol) % a.ncol < a.slots;
+        n0 = min(before * a.steps, a.K);
+        n1 = min(n0 + a.steps, a.K);
+        if (n0 >= n1) return;            // done (the whole cluster leaves)
+    }
     const int Oc = (int)(a.O >> clog);   // groups of this CTA, a multiple of blockDim.x
     const int nt = blockDim.x, t = threadIdx.x;
     int lo = 0;                          // flips below lo stay in this CTA
@@ -265,13 +278,18 @@ __global__ void __launch_bounds__(ResQSun<T, LG>::threads)
                 f.v[e] = KPM ? v.v[e] : mul_t(cK, v.v[e]);
             }
             if (!KPM) xb[c * Oc + ol] = v;
+            if (!KPM && n0 > 0) {   // b_{k+1} and b_{k+2} as the last launch left them
+                const Ch *w = reinterpret_cast<const Ch *>(a.state) + (((size_t)col * 2) * C + rank) * NCH * Oc + c * Oc + ol;
+                f = w[0];
+                z = w[(size_t)C * NCH * Oc];
+            }
             if (!KPM && a.K == 0) {
 #pragma unroll
                 for (int e = 0; e < W; ++e) a.Y[(int64_t)((outer << LG) + c * W + e) * a.yr + (int64_t)col * a.yc] = f.v[e];
             }
-            buf1[c * Oc + ol] = z;
-            buf0[c * Oc + ol] = f;
-            if (put) xch[(size_t)rank * NCH * Oc + c * Oc + ol] = f;
+            (n0 & 1 ? buf0 : buf1)[c * Oc + ol] = z;
+            (n0 & 1 ? buf1 : buf0)[c * Oc + ol] = f;
+            if (put) xch[(n0 & 1) * xpar + (size_t)rank * NCH * Oc + c * Oc + ol] = f;
         }
     }
     if constexpr (KPM) {
@@ -301,7 +319,7 @@ __global__ void __launch_bounds__(ResQSun<T, LG>::threads)
         }
     }
 
-    for (int n = 0; n < a.K; ++n) {
+    for (int n = n0; n < n1; ++n) {
         const Ch *q = (n & 1) ? buf1 : buf0;
         Ch *out = (n & 1) ? buf0 : buf1;
         const uint32_t qs = (n & 1) ? s1 : s0;
@@ -388,6 +406,13 @@ __global__ void __launch_bounds__(ResQSun<T, LG>::threads)
         }
     }
     column_sync(clog);   // no CTA leaves while another reads its rows
+    if (!KPM && n1 < a.K) {
+        Ch *w = reinterpret_cast<Ch *>(a.state) + (((size_t)col * 2) * C + rank) * NCH * Oc;
+        for (int i = t; i < NCH * Oc; i += nt) {
+            w[i] = (n1 & 1 ? buf1 : buf0)[i];
+            w[(size_t)C * NCH * Oc + i] = (n1 & 1 ? buf0 : buf1)[i];
+        }
+    }
     if constexpr (KPM) {
         if (a.K > 0 && t < 2) {
             double s = 0.0;
@@ -712,9 +737,10 @@ static bool qsun_plan(uint32_t O, int L_loc, int ncol, int clog, bool kpm, ResPl
     p->smem = (kpm ? 2 : 3) * block + Oc * sizeof(T) + ((p->threads / 32) * 4 + 2) * sizeof(double);
     p->kern = kpm ? (const void *)k_res_qsun<T, LG, true> : (const void *)k_res_qsun<T, LG, false>;
     const size_t far = clog * block;
-    p->work = far > kResFarShared ? 2 * (size_t)ncol * O * R::DG * sizeof(T) : 0;
+    p->far = far > kResFarShared;
+    p->work = p->far ? 2 * (size_t)ncol * O * R::DG * sizeof(T) : 0;
     p->busy_us = (double)block * (L_loc - clog + (kpm ? 3 : 4)) / 200e3 + far / 100e3;
-    p->us = p->busy_us + 0.5 + (p->work ? 0.9 : clog ? 0.5 : 0.0);
+    p->us = p->busy_us + 0.5 + (p->far ? 0.9 : clog ? 0.5 : 0.0);
     return p->smem <= kResSmem;
 }
 
@@ -828,11 +854,18 @@ static double step_us(const pf_op *op, int ncol, int elem, bool kpm) {
     return kpm ? 2 * us : us;
 }
 
+// A Quantum Sun filter of ncol columns with n < ncol clusters resident runs as
+// ncol launches of n columns and K / n steps each, every column resting in
+// ncol - n of them, so no launch leaves clusters idle: 2^16, s = 8, K = 430 on 7
+// clusters of 16 CTAs takes 8/7 rounds instead of two.  A launch costs about 10
+// us beyond its steps (its start, the vectors to memory and back).
+constexpr double kResSlotUs = 10.0;
+
 // Of the cluster sizes and widths that fit, the one with the least estimated
 // time for all columns: as many rounds of clusters as are not resident at once,
-// or the SMs' total work where that is more.
+// or the SMs' total work where that is more.  K: a filter's order.
 template <typename T>
-bool resident_plan(const pf_op *op, int ncol, bool kpm, ResPlan *best) {
+bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
     const double sms = op->h->num_sms;
     // KPM blocks of the step path hold 64 columns
     double bt = kpm ? step_us(op, std::min(ncol, 64), sizeof(T), true) * std::ceil(ncol / 64.0)
@@ -846,7 +879,16 @@ bool resident_plan(const pf_op *op, int ncol, bool kpm, ResPlan *best) {
             const int n = res_resident(p);
             if (n < 1) continue;
             const int groups = res_groups(p, ncol);
-            const double t = std::max((groups + n - 1) / n * p.us, groups * (1 << clog) * p.busy_us / sms);
+            double t = std::max((groups + n - 1) / n * p.us, groups * (1 << clog) * p.busy_us / sms);
+            if (op->kind == OP_QSUN && !kpm && groups > n) {
+                const int steps = (K + n - 1) / n;
+                const double ts = ncol * (steps * p.us + kResSlotUs) / std::max(K, 1);
+                if (ts < t) {
+                    t = ts;
+                    p.slots = n;
+                    p.work += 2 * (size_t)ncol * op->dim * sizeof(T);
+                }
+            }
             if (t < bt) {
                 bt = t;
                 *best = p;
@@ -908,7 +950,8 @@ static void res_launch(pf_op *op, const ResPlan &p, void *work, int ncol, cudaSt
     PF_CUDA(cudaFuncSetAttribute(p.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (op->kind == OP_QSUN) {
         a.O = (uint32_t)(op->dim >> op->L_grain);
-        a.xch = p.work ? static_cast<T *>(work) : nullptr;
+        a.xch = p.far ? static_cast<T *>(work) : nullptr;
+        a.state = static_cast<T *>(work) + (p.far ? 2 * (size_t)ncol * op->dim : 0);
         QSunDesc<T> d = res_qsun<T>(op);
         {
             const int dg = 1 << op->L_grain, W = std::min(dg, 16 / (int)sizeof(T)), ch = W * (int)sizeof(T);
@@ -920,6 +963,16 @@ static void res_launch(pf_op *op, const ResPlan &p, void *work, int ncol, cudaSt
             }
         }
         void *args[2] = {&d, &a};
+        if (p.slots > 0) {
+            cfg.gridDim = dim3((unsigned)p.slots << p.clog);
+            a.slots = p.slots;
+            a.steps = (a.K + p.slots - 1) / p.slots;
+            for (a.slot = 0; a.slot < ncol; ++a.slot) {
+                PF_CUDA(cudaLaunchKernelExC(&cfg, p.kern, args));
+                count_launches(1);
+            }
+            return;
+        }
         PF_CUDA(cudaLaunchKernelExC(&cfg, p.kern, args));
     } else {
         ResList<T> l{};
@@ -977,7 +1030,7 @@ void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &p, void *work, int 
 }
 
 #define PF_RES_INST(T)                                                                                              \
-    template bool resident_plan<T>(const pf_op *, int, bool, ResPlan *);                                           \
+    template bool resident_plan<T>(const pf_op *, int, bool, int, ResPlan *);                                         \
     template void resident_prepare<T>(pf_op *, cudaStream_t, const ResPlan &, void *);                             \
     template void resident_filter<T>(pf_op *, cudaStream_t, const ResPlan &, void *, int, int, const double *,     \
                                      double, double, const T *, int64_t, int64_t, T *, int64_t, int64_t);         \

@@ -166,8 +166,8 @@ static bool pinned_step(pf_op *op, int s, int elem) {
     return op->pinned_width.count(std::make_pair(elem, s)) > 0;
 }
 template <typename T>
-static bool resident_filter_plan(pf_op *op, int s, ResPlan *plan) {
-    return op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T)) && resident_plan<T>(op, s, false, plan);
+static bool resident_filter_plan(pf_op *op, int s, int K, ResPlan *plan) {
+    return op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T)) && resident_plan<T>(op, s, false, K, plan);
 }
 
 // Y = sum_k c_k T_k(Htilde) X on RI blocks (ClenshawAlgorithm.jl:12-29).
@@ -194,7 +194,7 @@ struct Filter {
     Filter(pf_op *op_, int s_, const std::vector<double> &coeffs, double a_, double b_, bool io = true,
            const void *list_ = nullptr)
         : op(op_), s(s_), K((int)coeffs.size() - 1), c(coeffs), a(a_), b(b_),
-          resident(io && resident_filter_plan<T>(op_, s_, &plan)), list(nullptr) {
+          resident(io && resident_filter_plan<T>(op_, s_, (int)coeffs.size() - 1, &plan)), list(nullptr) {
         const size_t n = (size_t)op->dim * s;
         if (resident) {
             dc.alloc(c.size());
@@ -324,7 +324,7 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
     // one on-chip recurrence per probe where a column fits a cluster (its dot
     // partials, 2^(clog + 4) bytes a probe and step, in at most 1 GB)
     ResPlan plan;
-    if ((int64_t)(M + 1) * R <= ((int64_t)1 << 22) && resident_plan<T>(op, R, true, &plan)) {
+    if ((int64_t)(M + 1) * R <= ((int64_t)1 << 22) && resident_plan<T>(op, R, true, M, &plan)) {
         DevArray<unsigned char> work(plan.work);
         DevArray<double> parts((size_t)2 * (M + 1) * R << plan.clog), rd((size_t)2 * (M + 1) * R);
         std::vector<double> hr((size_t)2 * (M + 1) * R);
@@ -1771,8 +1771,8 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     // is this solve's own CUDA graph of steps, whose kernel is tuned.
     pf_engine *eng = (h->engine && multi_eligible(op, fdtype)) ? h->engine : nullptr;
     ResPlan onchip;
-    const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, &onchip)
-                                                 : resident_filter_plan<float>(op, s, &onchip));
+    const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, (int)coeffs.size() - 1, &onchip)
+                                                 : resident_filter_plan<float>(op, s, (int)coeffs.size() - 1, &onchip));
     if (P->autotune && steps && (eng || !list || op->slab_cols > 0)) {
         bool have;
         {

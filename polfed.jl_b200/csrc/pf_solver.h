@@ -100,14 +100,16 @@ struct ResPlan {
     int cols = 1;         // columns per cluster
     int threads = 0;
     int rows = 0, groups = 0, list_smem = 0, x_smem = 0, diag_smem = 0;   // operators with neighbour lists
+    int far = 0, slots = 0;   // Quantum Sun: rows of other CTAs come from L2; columns per launch (0: all)
     size_t smem = 0;
     size_t work = 0;      // bytes of device workspace
     double us = 0, busy_us = 0;   // estimated time of a step of one cluster, and of that the time its SMs are busy
     const void *kern = nullptr;
 };
-// The plan for ncol columns of the operator; false: none (a column does not fit a cluster).
+// The plan for ncol columns of the operator (K: a filter's order); false: none
+// (a column does not fit a cluster, or the step kernels are estimated faster).
 template <typename T>
-bool resident_plan(const pf_op *op, int ncol, bool kpm, ResPlan *plan);
+bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *plan);
 // Fills the workspace (plan.work bytes) for the operator; once per workspace.
 template <typename T>
 void resident_prepare(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work);

@@ -89,6 +89,23 @@ def test_filter_equals_the_step_kernels(pkg, cuda, name, dtype):
         assert torch.equal(got, want), (K, float((got - want).abs().max()))
 
 
+@pytest.mark.parametrize("L_loc,L_grain,s,K", [(13, 3, 8, 203), (13, 3, 17, 120), (14, 3, 8, 64), (13, 2, 16, 301), (12, 4, 9, 150)])
+@pytest.mark.parametrize("dtype", ["fp64", "fp32"])
+def test_filter_of_more_columns_than_clusters(pkg, cuda, L_loc, L_grain, s, K, dtype):
+    """Large Quantum Sun columns run in several launches, each column resting in
+    some of them; orders that the launches do not divide."""
+    torch = cuda
+    op, ref = _qsun(pkg, L_loc, L_grain, 40), _qsun(pkg, L_loc, L_grain, 40)
+    tdt = torch.float64 if dtype == "fp64" else torch.float32
+    pkg.set_step_width(ref, s, 1, dtype)
+    X = _block(torch, op.dim, s, tdt, 6)
+    c = np.cos(np.arange(K + 1) * 0.8) / (K + 1)
+    got, want = torch.full_like(X, math.nan), torch.empty_like(X)
+    pkg.chebyshev_filter(op, got, X, c, 9.0, 0.3)
+    pkg.chebyshev_filter(ref, want, X, c, 9.0, 0.3)
+    assert torch.equal(got, want), float((got - want).abs().max())
+
+
 def test_filter_takes_strided_blocks(pkg, cuda):
     """Column-major blocks with padded columns, in place."""
     torch = cuda
