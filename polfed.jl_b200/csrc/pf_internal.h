@@ -276,6 +276,13 @@ template <typename T>
 void launch_chain_listed(pf_op *op, cudaStream_t st, const void *list, int s, const T *q, const T *p, const T *x, T *out,
                          double cx, double alpha, double beta, double inva, double shift, int flags, double *dots);
 
+// One step on column-major blocks of s >= 2 columns without staging
+// (pf_cm_step.cu): p and x both given (recurrence, final sum) or both null
+// (apply).  false: not offered for these arguments.
+template <typename T>
+bool launch_step_cm(pf_op *op, cudaStream_t st, int s, const T *q, const T *p, const T *x, T *out, int64_t ld,
+                    int64_t ldout, double cx, double alpha, double beta, double inva, double shift);
+
 // RI <-> column-major conversion, optional precision change.
 template <typename TS, typename TD>
 void launch_cm_to_ri(cudaStream_t st, int64_t D, int s, const TS *src, int64_t ld, TD *dst);
