@@ -18,7 +18,7 @@
 // CTAs' rows and the cluster barrier (about 500 clocks) on several.  Measured
 // on a B200, us a step of all columns, step kernels -> here (FP64): Quantum Sun
 // 2^11 s = 8 5.0 -> 1.6, 2^16 with 300 probes (KPM) 307 -> 151 for all; chain
-// L = 14 s = 1 6.9 -> 1.8, L = 16 s = 8 10.3 -> 4.0; CSR 6435 rows s = 4 4.5 -> 2.4.
+// L = 14 s = 1 6.9 -> 1.7, L = 16 s = 8 10.3 -> 3.2; CSR 6435 rows s = 4 4.5 -> 2.4.
 //
 // Every row is summed in the step kernels' order with the same explicitly
 // rounded operations (step_combine, fma_t), so results equal theirs bit for
@@ -54,10 +54,10 @@ struct ResArgs {
     // others), and the exchange inside the chunk
     uint32_t flip[PF_MAX_LOC];
     uint8_t inner[PF_MAX_LOC];
-    // Quantum Sun filters of more columns than clusters fit the device at once:
-    // `slots` > 0 launches of that many columns, each for `steps` steps
+    // filters of more columns (or groups of columns) than clusters fit the device
+    // at once: `slots` > 0 of them per launch, each for `steps` steps
     int slot, slots, steps;
-    T *state;            // [columns][2][D]: a column's vectors between its slots
+    T *state;            // their two vectors each, between their launches
     T *xch;              // exchange blocks [2][columns][D], or null: CTAs read each other's shared memory
 };
 
@@ -150,6 +150,20 @@ __device__ __forceinline__ Ch ld_l2(const Ch *p) {
     }
 }
 
+// The columns (or groups of columns, `groups` in all) of a rotating launch:
+// cluster i takes the i-th after the launch's first, from the step n0 its
+// earlier launches reached to n1.  false: it is done (the whole cluster leaves).
+template <typename T>
+__device__ __forceinline__ bool res_slot(const ResArgs<T> &a, int groups, int *grp, int *n0, int *n1) {
+    const int g = (*grp + a.slot) % groups;
+    int before = 0;
+    for (int j = 0; j < a.slot; ++j) before += (g - j + groups) % groups < a.slots;
+    *grp = g;
+    *n0 = min(before * a.steps, a.K);
+    *n1 = min(*n0 + a.steps, a.K);
+    return *n0 < *n1;
+}
+
 // The sum over the column's threads of v, the same in every one of them.
 // red: one double per warp plus one.
 __device__ double column_sum(double v, double *red, int clog) {
@@ -225,14 +239,7 @@ __global__ void __launch_bounds__(ResQSun<T, LG>::threads)
     const uint32_t rank = clog ? cluster_rank() : 0u;
     int col = blockIdx.x >> clog;
     int n0 = 0, n1 = a.K;                // steps of this launch
-    if (!KPM && a.slots > 0) {
-        col = (col + a.slot) % a.ncol;
-        int before = 0;                  // earlier launches with this column
-        for (int j = 0; j < a.slot; ++j) before += (col - j + a.ncol) % a.ncol < a.slots;
-        n0 = min(before * a.steps, a.K);
-        n1 = min(n0 + a.steps, a.K);
-        if (n0 >= n1) return;            // done (the whole cluster leaves)
-    }
+    if (!KPM && a.slots > 0 && !res_slot(a, a.ncol, &col, &n0, &n1)) return;
     const int Oc = (int)(a.O >> clog);   // groups of this CTA, a multiple of blockDim.x
     const int nt = blockDim.x, t = threadIdx.x;
     int lo = 0;                          // flips below lo stay in this CTA
@@ -699,6 +706,106 @@ __global__ void __launch_bounds__(kResListThreads)
     }
 }
 
+// The filter of a chain whose CTAs hold at most a row per thread: a thread's
+// list stays in registers as ready addresses, with its X, its diagonal and its
+// own values, so a step is one barrier, its gathers (eight in flight) and their
+// sum.  us a step, k_res_list -> here: XXZ L = 14 s = 1 1.76 -> 1.69, L = 16 s = 1
+// 3.07 -> 2.47, s = 8 3.99 -> 3.16.  More than 24 entries or 1024 rows a CTA do
+// not fit its 64 registers a thread: those stay with k_res_list.
+template <typename T, int V, int G>
+__global__ void __launch_bounds__(1024)
+    k_res_pinned(const __grid_constant__ ResList<T> l, const __grid_constant__ ResArgs<T> a) {
+    using Ch = Pack<T, V>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int clog = a.clog;
+    const uint32_t rank = clog ? cluster_rank() : 0u;
+    int grp = blockIdx.x >> clog, n0 = 0, n1 = a.K;
+    if (a.slots > 0 && !res_slot(a, (a.ncol + V - 1) / V, &grp, &n0, &n1)) return;
+    const int col0 = grp * V, nv = min(V, a.ncol - col0);
+    const int t = threadIdx.x, R = l.rows;
+    const uint32_t row = rank * (uint32_t)R + t;
+    const bool mine = t < R && row < l.D;
+    const int lbits = 16 - clog;
+    Ch *buf0 = reinterpret_cast<Ch *>(smem_raw), *buf1 = buf0 + R;
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(buf0), s1 = (uint32_t)__cvta_generic_to_shared(buf1);
+    uint32_t at[8 * G], on = 0u;
+    Ch x, qo, po;
+    T dg = T(0);
+    const T cK = (T)__ldg(a.coef + a.K);
+#pragma unroll
+    for (int e = 0; e < V; ++e) x.v[e] = qo.v[e] = po.v[e] = T(0);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        uint4 w = make_uint4(~0u, ~0u, ~0u, ~0u);
+        if (mine) w = __ldg(l.ent + (size_t)g * l.D + row);
+        const uint32_t w4[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t e = (w4[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+            if (e != kResNone) on |= 1u << (8 * g + u);
+            at[8 * g + u] = (clog ? map_rank(s0, e >> lbits) : s0) + (e & ((1u << lbits) - 1u)) * (uint32_t)sizeof(Ch);
+        }
+    }
+    if (mine) {
+        dg = __ldg(l.diag + row);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            if (e < nv) x.v[e] = __ldg(a.X + (int64_t)row * a.xr + (int64_t)(col0 + e) * a.xc);
+            qo.v[e] = mul_t(cK, x.v[e]);
+            if (a.K == 0 && e < nv) a.Y[(int64_t)row * a.yr + (int64_t)(col0 + e) * a.yc] = qo.v[e];
+        }
+    }
+    Ch *state = reinterpret_cast<Ch *>(a.state) + ((size_t)(2 * grp) << clog) * R + rank * (uint32_t)R + t;   // then po
+    const size_t spo = (size_t)R << clog;
+    if (mine && n0 > 0) {
+        qo = state[0];
+        po = state[spo];
+    }
+    if (mine) (n0 & 1 ? buf1 : buf0)[t] = qo;
+    T ck = a.K == 0 ? T(0) : (T)__ldg(a.coef + a.K - 1 - n0);
+    for (int n = n0; n < n1; ++n) {
+        const uint32_t dq = (n & 1) ? s1 - s0 : 0u;
+        Ch *out = (n & 1) ? buf0 : buf1;
+        const bool last = n == a.K - 1;
+        const T alpha = last ? T(1) : T(2);
+        const T cnext = last ? T(0) : (T)__ldg(a.coef + a.K - 2 - n);
+        column_sync(clog);
+        Ch v;
+        T acc[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[e] = T(0);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            Ch f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) f[u] = ld_shared_if<Ch, true>(at[8 * g + u] + dq, (on >> (8 * g + u)) & 1u);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int e = 0; e < V; ++e) acc[e] = fma_t(l.jhalf[8 * g + u], f[u].v[e], acc[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            v.v[e] = step_combine<T>(true, true, true, ck, x.v[e], alpha, acc[e], dg, qo.v[e], a.inva, a.boa, T(-1), po.v[e]);
+            po.v[e] = qo.v[e];
+            qo.v[e] = v.v[e];
+        }
+        if (mine && last) {
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+                if (e < nv) a.Y[(int64_t)row * a.yr + (int64_t)(col0 + e) * a.yc] = v.v[e];
+        } else if (mine) {
+            out[t] = v;
+        }
+        ck = cnext;
+    }
+    column_sync(clog);   // no CTA leaves while another reads its rows
+    if (mine && n1 < a.K) {
+        state[0] = qo;
+        state[spo] = po;
+    }
+}
+
 // out[(m * 2 + v) * ncol + c] = the sum over a column's CTAs of its partial dots, in rank order
 __global__ void k_res_dots(const double *__restrict__ part, int64_t n, int C, int ncol, double *__restrict__ out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -762,6 +869,12 @@ static const void *list_kernel(bool csr, bool kpm) {
     return kpm ? (const void *)k_res_list<T, V, false, true> : (const void *)k_res_list<T, V, false, false>;
 }
 
+template <typename T, int V>
+static const void *pinned_kernel(int groups) {
+    return groups == 1 ? (const void *)k_res_pinned<T, V, 1> : groups == 2 ? (const void *)k_res_pinned<T, V, 2>
+                                                             : (const void *)k_res_pinned<T, V, 3>;
+}
+
 // Entries of a row of a chain or CSR operator, on average.
 static double list_terms(const pf_op *op) {
     if (op->kind == OP_CSR) return (double)op->nnz / (double)op->dim;
@@ -803,6 +916,20 @@ static bool list_plan(const pf_op *op, int V, int clog, bool kpm, ResPlan *p) {
     const double wide = V * (int)sizeof(T) == 16 ? 1.25 : V * (int)sizeof(T) == 4 ? 0.85 : 1.0;
     p->busy_us = (double)rows * list_terms(op) * (clog ? 0.27e-3 : 0.18e-3) * wide * (csr ? 1.25 : 1.0);
     p->us = p->busy_us + (clog ? 1.2 : 0.4);
+    if (!csr && !kpm && p->groups <= 3 && rows <= 1024) {
+        // measured: 1.35 us for the barrier and the latency of remote rows, 0.042
+        // ns a row and entry for every doubling of the CTAs (the remote share
+        // grows so); in one CTA 0.35 us and 0.1 ns
+        const double size = V * (int)sizeof(T) == 16 ? 1.9 : V * (int)sizeof(T) == 4 ? 0.7 : 1.0;
+        p->busy_us = (double)rows * list_terms(op) * (clog ? 0.042e-3 * clog * size : 0.1e-3 * wide);
+        p->us = p->busy_us + (clog ? 1.35 : 0.35);
+        p->threads = (int)(rows + 31) / 32 * 32;
+        p->smem = 2 * vec;
+        p->pinned = 1;
+        if constexpr (sizeof(T) == 8) p->kern = V == 1 ? pinned_kernel<T, 1>(p->groups) : pinned_kernel<T, 2>(p->groups);
+        else p->kern = V == 1 ? pinned_kernel<T, 1>(p->groups) : V == 2 ? pinned_kernel<T, 2>(p->groups) : pinned_kernel<T, 4>(p->groups);
+        return true;
+    }
     if constexpr (sizeof(T) == 8) p->kern = V == 1 ? list_kernel<T, 1>(csr, kpm) : list_kernel<T, 2>(csr, kpm);
     else p->kern = V == 1 ? list_kernel<T, 1>(csr, kpm) : V == 2 ? list_kernel<T, 2>(csr, kpm) : list_kernel<T, 4>(csr, kpm);
     return true;
@@ -854,11 +981,11 @@ static double step_us(const pf_op *op, int ncol, int elem, bool kpm) {
     return kpm ? 2 * us : us;
 }
 
-// A Quantum Sun filter of ncol columns with n < ncol clusters resident runs as
-// ncol launches of n columns and K / n steps each, every column resting in
-// ncol - n of them, so no launch leaves clusters idle: 2^16, s = 8, K = 430 on 7
-// clusters of 16 CTAs takes 8/7 rounds instead of two.  A launch costs about 10
-// us beyond its steps (its start, the vectors to memory and back).
+// A filter of g columns (or groups of columns) with n < g clusters resident runs
+// as g launches of n of them and K / n steps each, every one resting in g - n
+// launches, so no launch leaves clusters idle: eight columns on 7 clusters of 16
+// CTAs take 8/7 rounds instead of two.  A launch costs about 10 us beyond its
+// steps (its start, the vectors to memory and back).
 constexpr double kResSlotUs = 10.0;
 
 // Of the cluster sizes and widths that fit, the one with the least estimated
@@ -880,13 +1007,14 @@ bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
             if (n < 1) continue;
             const int groups = res_groups(p, ncol);
             double t = std::max((groups + n - 1) / n * p.us, groups * (1 << clog) * p.busy_us / sms);
-            if (op->kind == OP_QSUN && !kpm && groups > n) {
+            if ((op->kind == OP_QSUN || p.pinned) && !kpm && K > 0 && groups > n) {
                 const int steps = (K + n - 1) / n;
-                const double ts = ncol * (steps * p.us + kResSlotUs) / std::max(K, 1);
+                const double ts = groups * (steps * p.us + kResSlotUs) / std::max(K, 1);
                 if (ts < t) {
                     t = ts;
                     p.slots = n;
-                    p.work += 2 * (size_t)ncol * op->dim * sizeof(T);
+                    p.work += 2 * (size_t)groups * p.cols * sizeof(T) *
+                              (p.pinned ? (size_t)p.rows << p.clog : (size_t)op->dim);
                 }
             }
             if (t < bt) {
@@ -940,6 +1068,21 @@ void resident_prepare(pf_op *op, cudaStream_t st, const ResPlan &p, void *work) 
     count_launches(1);
 }
 
+// The launch, or the plan's rotating launches.  args: the kernel's, with &a.
+template <typename T>
+static void res_launch_slots(cudaLaunchConfig_t &cfg, const ResPlan &p, void **args, ResArgs<T> &a, int ncol) {
+    const int launches = p.slots > 0 ? res_groups(p, ncol) : 1;
+    if (p.slots > 0) {
+        cfg.gridDim = dim3((unsigned)p.slots << p.clog);
+        a.slots = p.slots;
+        a.steps = (a.K + p.slots - 1) / p.slots;
+    }
+    for (a.slot = 0; a.slot < launches; ++a.slot) {
+        PF_CUDA(cudaLaunchKernelExC(&cfg, p.kern, args));
+        count_launches(1);
+    }
+}
+
 template <typename T>
 static void res_launch(pf_op *op, const ResPlan &p, void *work, int ncol, cudaStream_t st, ResArgs<T> &a) {
     a.clog = p.clog;
@@ -963,17 +1106,7 @@ static void res_launch(pf_op *op, const ResPlan &p, void *work, int ncol, cudaSt
             }
         }
         void *args[2] = {&d, &a};
-        if (p.slots > 0) {
-            cfg.gridDim = dim3((unsigned)p.slots << p.clog);
-            a.slots = p.slots;
-            a.steps = (a.K + p.slots - 1) / p.slots;
-            for (a.slot = 0; a.slot < ncol; ++a.slot) {
-                PF_CUDA(cudaLaunchKernelExC(&cfg, p.kern, args));
-                count_launches(1);
-            }
-            return;
-        }
-        PF_CUDA(cudaLaunchKernelExC(&cfg, p.kern, args));
+        res_launch_slots(cfg, p, args, a, ncol);
     } else {
         ResList<T> l{};
         uint16_t *ent;
@@ -992,10 +1125,10 @@ static void res_launch(pf_op *op, const ResPlan &p, void *work, int ncol, cudaSt
             l.diag = d.diag;
             for (int b = 0; b < d.nb; ++b) l.jhalf[b] = d.jhalf[b];
         }
+        a.state = val;   // a rotating chain filter's vectors, in the place of CSR values
         void *args[2] = {&l, &a};
-        PF_CUDA(cudaLaunchKernelExC(&cfg, p.kern, args));
+        res_launch_slots(cfg, p, args, a, ncol);
     }
-    count_launches(1);
 }
 
 template <typename T>

@@ -100,7 +100,9 @@ struct ResPlan {
     int cols = 1;         // columns per cluster
     int threads = 0;
     int rows = 0, groups = 0, list_smem = 0, x_smem = 0, diag_smem = 0;   // operators with neighbour lists
-    int far = 0, slots = 0;   // Quantum Sun: rows of other CTAs come from L2; columns per launch (0: all)
+    int far = 0;          // Quantum Sun: rows of other CTAs come from L2
+    int pinned = 0;       // chains: a row per thread, its list in registers
+    int slots = 0;        // groups of columns per launch (0: all in one)
     size_t smem = 0;
     size_t work = 0;      // bytes of device workspace
     double us = 0, busy_us = 0;   // estimated time of a step of one cluster, and of that the time its SMs are busy

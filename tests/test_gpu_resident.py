@@ -106,6 +106,22 @@ def test_filter_of_more_columns_than_clusters(pkg, cuda, L_loc, L_grain, s, K, d
     assert torch.equal(got, want), float((got - want).abs().max())
 
 
+@pytest.mark.parametrize("L,s,K", [(16, 8, 200), (16, 15, 131), (16, 9, 0), (12, 3, 64), (14, 40, 90), (17, 3, 50)])
+@pytest.mark.parametrize("dtype", ["fp64", "fp32"])
+def test_chain_filter_with_a_row_per_thread(pkg, cuda, L, s, K, dtype):
+    """Lists in registers, in one launch and in rotating ones."""
+    torch = cuda
+    op, ref = _chain(pkg, L, L // 2, 41, uniform=False), _chain(pkg, L, L // 2, 41, uniform=False)
+    tdt = torch.float64 if dtype == "fp64" else torch.float32
+    pkg.set_step_width(ref, s, 1, dtype)
+    X = _block(torch, op.dim, s, tdt, 6)
+    c = np.cos(np.arange(K + 1) * 0.8) / (K + 1)
+    got, want = torch.full_like(X, math.nan), torch.empty_like(X)
+    pkg.chebyshev_filter(op, got, X, c, 11.0, 0.3)
+    pkg.chebyshev_filter(ref, want, X, c, 11.0, 0.3)
+    assert torch.equal(got, want), float((got - want).abs().max())
+
+
 def test_filter_takes_strided_blocks(pkg, cuda):
     """Column-major blocks with padded columns, in place."""
     torch = cuda
