@@ -136,6 +136,7 @@ struct pf_handle {
     // (the two extremal Lanczos probes); created on first use
     pf_handle *aux = nullptr;
     std::mutex aux_mu;
+    bool shared = false;              // a worker of a pool of several: other solves run beside this one's
     // filter engine of the pool this handle works for (not owned); null: the
     // handle runs its own graph-captured filters
     pf_engine *engine = nullptr;

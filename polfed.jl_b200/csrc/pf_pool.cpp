@@ -244,6 +244,7 @@ pf_pool *pool_create(int device, int workers, double budget) {
             t_new_handle_priority = saved;
             if (st != PF_OK) throw Error(PF_ERR_CUDA, pf_last_error());
             pool->urgent.push_back(h);
+            pool->handles[w]->shared = pool->urgent[w]->shared = workers > 1;
         }
         if (budget <= 0) {
             // read after the handles exist; each of the 2 W handles later grows

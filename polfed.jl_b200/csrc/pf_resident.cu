@@ -985,7 +985,11 @@ static double step_us(const pf_op *op, int ncol, int elem, bool kpm) {
 // as g launches of n of them and K / n steps each, every one resting in g - n
 // launches, so no launch leaves clusters idle: eight columns on 7 clusters of 16
 // CTAs take 8/7 rounds instead of two.  A launch costs about 10 us beyond its
-// steps (its start, the vectors to memory and back).
+// steps (its start, the vectors to memory and back).  A chain's filter beside
+// others in a pool does not rotate: two columns a cluster then take half the
+// clusters for 12 % more time each, and the others run on the rest (eight XXZ L =
+// 16 solves in flight 511 ms rotating, 390 not; the Quantum Sun's CTAs hold one
+// column only).
 constexpr double kResSlotUs = 10.0;
 
 // Of the cluster sizes and widths that fit, the one with the least estimated
@@ -1007,7 +1011,8 @@ bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
             if (n < 1) continue;
             const int groups = res_groups(p, ncol);
             double t = std::max((groups + n - 1) / n * p.us, groups * (1 << clog) * p.busy_us / sms);
-            if ((op->kind == OP_QSUN || p.pinned) && !kpm && K > 0 && groups > n) {
+            const bool rotates = op->kind == OP_QSUN || (p.pinned && !op->h->shared);
+            if (rotates && !kpm && K > 0 && groups > n) {
                 const int steps = (K + n - 1) / n;
                 const double ts = groups * (steps * p.us + kResSlotUs) / std::max(K, 1);
                 if (ts < t) {
