@@ -163,12 +163,6 @@ static void launch_cm(pf_op *op, cudaStream_t st, const ChainDesc<T> &ch, const 
     else launch_cm<T>(op, st, cs, a, 0);
 }
 
-// Whether [a, a + na) and [b, b + nb) overlap.
-static bool overlap(const void *a, size_t na, const void *b, size_t nb) {
-    const char *x = static_cast<const char *>(a), *y = static_cast<const char *>(b);
-    return x < y + nb && y < x + na;
-}
-
 template <typename T>
 bool launch_step_cm(pf_op *op, cudaStream_t st, int s, const T *q, const T *p, const T *x, T *out, int64_t ld,
                     int64_t ldout, double cx, double alpha, double beta, double inva, double shift) {

@@ -115,6 +115,12 @@ __host__ __device__ inline int rank_table_offset(int c) {
     return n;
 }
 
+// Whether [a, a + na) and [b, b + nb) overlap.
+inline bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+    const char *x = static_cast<const char *>(a), *y = static_cast<const char *>(b);
+    return x < y + nb && y < x + na;
+}
+
 }  // namespace pf
 
 // ------------------------------------------------------------ opaque handles

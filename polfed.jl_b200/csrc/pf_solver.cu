@@ -1542,6 +1542,31 @@ void op_gram_bf16x3(pf_handle *h, int64_t D, int nB, const double *B, int64_t ld
 }
 
 // ------------------------------------------------------- op-level filter
+template <typename T>
+static void op_filter(pf_op *op, double a, double b, const std::vector<double> &c, int s, const T *X, int64_t ldx, T *Y,
+                      int64_t ldy) {
+    cudaStream_t st = op->h->stream;
+    const int64_t D = op->dim;
+    Filter<T> f(op, s, c, a, b);
+    // On chip a column's output may be written while others still read X: X
+    // itself may be the output (an element is read, then written, by one
+    // thread), other overlaps are staged.
+    const bool apart = (X == Y && ldx == ldy) || !overlap(X, ((size_t)(s - 1) * ldx + D) * sizeof(T), Y,
+                                                          ((size_t)(s - 1) * ldy + D) * sizeof(T));
+    if (f.resident && apart) {
+        f.run_resident(st, X, 1, ldx, Y, 1, ldy);
+    } else {
+        launch_cm_to_ri<T, T>(st, D, s, X, ldx, f.x());
+        if (f.resident) {
+            f.run_resident(st, f.x(), s, 1, Y, 1, ldy);
+        } else {
+            f.enqueue(st);
+            launch_ri_to_cm<T, T>(st, D, s, f.Y.p, Y, ldy);
+        }
+    }
+    sync(op->h);
+}
+
 void op_filter(pf_op *op, int dtype, double a, double b, int K, const double *coeffs, int s, const void *X,
                int64_t ldx, void *Y, int64_t ldy) {
     PF_CHECK(coeffs && X && Y && K >= 0 && s >= 1, PF_ERR_INVALID, "invalid filter arguments");
@@ -1549,32 +1574,10 @@ void op_filter(pf_op *op, int dtype, double a, double b, int K, const double *co
     PF_CHECK(a != 0.0 && std::isfinite(a) && std::isfinite(b), PF_ERR_INVALID, "rescaling a must be finite and nonzero");
     PF_CUDA(cudaSetDevice(op->h->device));
     AllocStream alloc_guard(op->h->stream);
-    std::vector<double> c(coeffs, coeffs + K + 1);
-    cudaStream_t st = op->h->stream;
-    const int64_t D = op->dim;
-    if (dtype == PF_F64) {
-        Filter<double> f(op, s, c, a, b);
-        if (f.resident) {
-            f.run_resident(st, (const double *)X, 1, ldx, (double *)Y, 1, ldy);
-            sync(op->h);
-            return;
-        }
-        launch_cm_to_ri<double, double>(st, D, s, (const double *)X, ldx, f.X.p);
-        f.enqueue(st);
-        launch_ri_to_cm<double, double>(st, D, s, f.Y.p, (double *)Y, ldy);
-        sync(op->h);
-    } else if (dtype == PF_F32) {
-        Filter<float> f(op, s, c, a, b);
-        if (f.resident) {
-            f.run_resident(st, (const float *)X, 1, ldx, (float *)Y, 1, ldy);
-            sync(op->h);
-            return;
-        }
-        launch_cm_to_ri<float, float>(st, D, s, (const float *)X, ldx, f.X.p);
-        f.enqueue(st);
-        launch_ri_to_cm<float, float>(st, D, s, f.Y.p, (float *)Y, ldy);
-        sync(op->h);
-    } else throw Error(PF_ERR_INVALID, "dtype must be PF_F64 or PF_F32");
+    const std::vector<double> c(coeffs, coeffs + K + 1);
+    if (dtype == PF_F64) op_filter<double>(op, a, b, c, s, (const double *)X, ldx, (double *)Y, ldy);
+    else if (dtype == PF_F32) op_filter<float>(op, a, b, c, s, (const float *)X, ldx, (float *)Y, ldy);
+    else throw Error(PF_ERR_INVALID, "dtype must be PF_F64 or PF_F32");
 }
 
 void op_kpm(pf_op *op, int dtype, double a, double b, int N, int R, const void *probes, int64_t ldp, int probe_kind,

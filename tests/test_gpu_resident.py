@@ -122,6 +122,26 @@ def test_chain_filter_with_a_row_per_thread(pkg, cuda, L, s, K, dtype):
     assert torch.equal(got, want), float((got - want).abs().max())
 
 
+@pytest.mark.parametrize("kind", ["chain", "qsun"])
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_filter_output_over_its_input(pkg, cuda, kind, shift):
+    """Y over X: the same block, one starting a column later, one two rows later."""
+    torch = cuda
+    op = _chain(pkg, 12, 6, 41, uniform=False) if kind == "chain" else _qsun(pkg, 8, 3, 5)
+    D, s, K = op.dim, 12, 40
+    X = _block(torch, D, s, torch.float64, 9)
+    c = np.cos(np.arange(K + 1) * 0.8) / (K + 1)
+    want = torch.empty_like(X)
+    pkg.chebyshev_filter(op, want, X, c, 11.0, 0.3)
+    at = (0, D, 2)[shift]
+    base = torch.zeros((s + 1) * D, dtype=torch.float64, device=X.device)
+    Xv = base[: s * D].view(s, D).t()
+    Yv = base[at : at + s * D].view(s, D).t()
+    Xv.copy_(X)
+    pkg.chebyshev_filter(op, Yv, Xv, c, 11.0, 0.3)
+    assert torch.equal(Yv, want)
+
+
 def test_filter_takes_strided_blocks(pkg, cuda):
     """Column-major blocks with padded columns, in place."""
     torch = cuda
