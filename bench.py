@@ -51,7 +51,7 @@ WORKLOAD = {
     "target": "(:rescaled, 0.5)", "dos_N": 250, "dos_R": 300, "kernel": "Jackson", "eigentol": 1e-10,
 }
 L2_FLUSH_BYTES = 256 << 20  # > 126 MB L2
-PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "k_step_qsun_fp64_D65536_s8.md")
+PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "k_res_qsun_fp64_D65536_s8.md")
 
 
 def _env_int(name, default):
@@ -172,7 +172,8 @@ def read_peaks():
 
 
 def read_traffic():
-    """DRAM bytes per launch of the step kernel from the committed ncu summary."""
+    """DRAM bytes per launch from the committed ncu summary, if it names them (a
+    filter on chip moves its blocks once, not per step)."""
     try:
         text = open(PROFILE_SUMMARY).read()
     except OSError:
@@ -413,17 +414,17 @@ def run_ours(args, rank, world, local_rank):
         "single_solve": {"value": single_value, "unit": "eigenpairs/s",
                          "note": "one solve at a time on one stream (the plain single-solve form)"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "k_step (Clenshaw recurrence)", "achieved": achieved,
+        "roofline": {"bound": "hbm", "kernel": "k_res_qsun (Clenshaw recurrence on chip, per step)", "achieved": achieved,
                      "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": read_traffic(), "algorithmic_bytes_per_launch": alg_bytes,
                      "avg_launch_us": avg_step * 1e6,
                      "measured_in": "the single-solve runs (library CUDA-event stage timers)",
                      "l2_gather": {"peak_gbs": gather_peak, "achieved_gbs": flip_bytes / avg_step / 1e9,
                                    "frac": flip_bytes / avg_step / 1e9 / gather_peak,
-                                   "note": "the step's blocks stay in L2 (3 x 4 MB); its L_loc flipped-row "
-                                           "gathers (64 B each) against the measured random-row gather "
+                                   "note": "the step's columns stay in shared memory, so its L_loc flipped-row "
+                                           "reads (64 B each) may exceed the measured random-row gather "
                                            "throughput of an L2-resident block (pf_gather_peak)"},
-                     "kpm": {"kernel": "k_step (KPM doubling step, fused dots)",
+                     "kpm": {"kernel": "k_res_qsun (KPM doubling steps on chip, dots fused)",
                              "algorithmic_bytes_per_solve": kpm_bytes,
                              "achieved": kpm_bytes / kpm_sec / 1e9, "frac": kpm_bytes / kpm_sec / 1e9 / peak,
                              "seconds_per_solve": kpm_sec,
