@@ -147,12 +147,16 @@ static void launch_cm(pf_op *op, cudaStream_t st, const Desc &d, const CmArgs<T>
     count_launches(1);
 }
 
+// Columns per thread.  Few rows: one, for more threads; else as many as share a row's flips at no loss.
+static int cm_columns(int64_t D, int s) { return D * s <= 100000 ? 1 : s == 2 ? 2 : 4; }
+
 template <typename T, class Desc>
 static void launch_cm(pf_op *op, cudaStream_t st, const Desc &d, const CmArgs<T> &a, int smem) {
-    // few rows: a column per thread, for more threads; else as many columns as share a row's flips at no loss
-    if ((int64_t)a.D * a.s <= 100000) launch_cm<T, 1, Desc>(op, st, d, a, smem);
-    else if (a.s == 2) launch_cm<T, 2, Desc>(op, st, d, a, smem);
-    else launch_cm<T, 4, Desc>(op, st, d, a, smem);
+    switch (cm_columns(a.D, a.s)) {
+        case 1: launch_cm<T, 1, Desc>(op, st, d, a, smem); break;
+        case 2: launch_cm<T, 2, Desc>(op, st, d, a, smem); break;
+        default: launch_cm<T, 4, Desc>(op, st, d, a, smem);
+    }
 }
 
 template <typename T>
@@ -167,7 +171,8 @@ template <typename T>
 bool launch_step_cm(pf_op *op, cudaStream_t st, int s, const T *q, const T *p, const T *x, T *out, int64_t ld,
                     int64_t ldout, double cx, double alpha, double beta, double inva, double shift) {
     const int64_t D = op->dim;
-    if (s < 2 || s > 8 * 65535 || (op->kind == OP_CHAIN && op->chain64.diag == nullptr)) return false;
+    if (s < 2 || (op->kind == OP_CHAIN && op->chain64.diag == nullptr)) return false;
+    if ((s - 1) / cm_columns(D, s) >= 65535) return false;   // more blocks of columns than a grid's second dimension has
     // Where copies and row gathers are faster: wide blocks of many rows, whose
     // gathers fill whole sectors only in the row-interleaved layout (J1-J2 L = 22,
     // s = 8 FP64: 254 us staged, 355 here; Quantum Sun 2^18, s = 24: 148 and 170).

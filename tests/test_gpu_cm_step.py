@@ -73,3 +73,27 @@ def test_apply_in_place(pkg, cuda, ops):
     pkg.apply(op, want, X, 2.0, 0.1)
     pkg.apply(op, X, X, 2.0, 0.1)
     assert torch.equal(X, want)
+
+
+@pytest.mark.parametrize("kind,s", [("chain", 65535), ("chain", 70000), ("qsun", 262140), ("qsun", 300001)])
+def test_more_columns_than_a_launch_has_column_blocks(pkg, cuda, kind, s):
+    """Very wide blocks of a handful of states: a chain with one state, 65536
+    and more columns of one thread each; a Quantum Sun with four, 262144 and more
+    of four columns a thread.  Against two calls of half the columns."""
+    torch = cuda
+    rng = np.random.default_rng(8)
+    if kind == "chain":
+        op = pkg.SpinChainOperator(5, 0, pkg.chain_bonds(5, 1), rng.random(5), rng.random(5), rng.random(5))
+    else:
+        f, n, c, g = pkg.qsun_parameters(1, 1, 0.75, rng=rng)
+        op = pkg.QSunOperator(1, 1, 0.9, c, n, f, g)
+    q, p, x = (_padded(torch, op.dim, s, 0, torch.float64, k) for k in range(3))
+    for call in ("apply", "recurrence"):
+        def run(c0, c1):
+            out = torch.empty_like(q[:, c0:c1].t().contiguous().t())
+            a = [t[:, c0:c1] for t in (q, p, x)]
+            if call == "apply":
+                return pkg.apply(op, out, a[0], 3.0, 0.2)
+            return pkg.clenshaw_recurrence(op, out, a[0], a[1], 0.7, a[2], 3.0, 0.2)
+        h = s // 2
+        assert torch.equal(run(0, s), torch.cat([run(0, h), run(h, s)], dim=1))
