@@ -47,7 +47,8 @@ struct ResArgs {
     T inva, boa;
     int probe_kind;
     uint64_t seed;
-    int ncol;            // KPM: columns
+    int ncol;            // columns of the launch
+    int col0;            // KPM: number of the first of them, for drawn probes
     double *part;        // KPM: [K + 1][ncol][2^clog][2] dot partials
     // Quantum Sun, by outer spin: the XOR of a chunk's byte offset in a CTA's
     // block (spins of the CTA's own range) or of its chunk part alone (the
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(ResQSun<T, LG>::threads)
             for (int e = 0; e < W; ++e) {
                 const uint32_t row = (outer << LG) + c * W + e;
                 if (!KPM || a.X) v.v[e] = __ldg(a.X + (int64_t)row * a.xr + (int64_t)col * a.xc);
-                else v.v[e] = (T)probe_value(a.probe_kind, a.seed, row, col);
+                else v.v[e] = (T)probe_value(a.probe_kind, a.seed, row, a.col0 + col);
                 nrm += (double)v.v[e] * (double)v.v[e];
                 z.v[e] = T(0);
                 f.v[e] = KPM ? v.v[e] : mul_t(cK, v.v[e]);
@@ -559,7 +560,7 @@ __global__ void __launch_bounds__(kResListThreads)
         if (!KPM || a.X) v = load_x(row);
         else {
 #pragma unroll
-            for (int e = 0; e < V; ++e) v.v[e] = (T)probe_value(a.probe_kind, a.seed, row, col0 + e);
+            for (int e = 0; e < V; ++e) v.v[e] = (T)probe_value(a.probe_kind, a.seed, row, a.col0 + col0 + e);
         }
 #pragma unroll
         for (int e = 0; e < V; ++e) {
@@ -845,7 +846,9 @@ static bool qsun_plan(uint32_t O, int L_loc, int ncol, int clog, bool kpm, ResPl
     p->kern = kpm ? (const void *)k_res_qsun<T, LG, true> : (const void *)k_res_qsun<T, LG, false>;
     const size_t far = clog * block;
     p->far = far > kResFarShared;
-    p->work = p->far ? 2 * (size_t)ncol * O * R::DG * sizeof(T) : 0;
+    const size_t exchange = p->far ? 2 * (size_t)O * R::DG * sizeof(T) : 0;   // of a column
+    p->work = kpm ? 0 : (size_t)ncol * exchange;
+    p->work_col = exchange;
     p->busy_us = (double)block * (L_loc - clog + (kpm ? 3 : 4)) / 200e3 + far / 100e3;
     p->us = p->busy_us + 0.5 + (p->far ? 0.9 : clog ? 0.5 : 0.0);
     return p->smem <= kResSmem;
@@ -992,9 +995,26 @@ static double step_us(const pf_op *op, int ncol, int elem, bool kpm) {
 // column only).
 constexpr double kResSlotUs = 10.0;
 
+// A KPM run takes its columns in launches of whole rounds of clusters, so many
+// that the columns' exchange blocks and dot partials stay below kResKpmBytes or
+// the two blocks of 64 columns the step kernels would hold, whichever is more
+// (a round's exchange blocks are at most the SMs' shared memory twice).  A
+// launch's last round waits for its slowest cluster: the Quantum Sun 2^16 with
+// 300 probes takes 18.32 ms in one launch, 18.49 in two, 18.69 in the six of 67
+// MB.  false: not even a round fits.
+static bool kpm_launch(ResPlan *p, int64_t D, int elem, int ncol, int M, int resident) {
+    const double each = (double)p->work_col + 16.0 * (M + 1) * (1 << p->clog);
+    const double room = std::max((double)kResKpmBytes, 2.0 * (double)D * 64 * elem);
+    const int64_t fit = (int64_t)std::min(room / each, 1e9), round = (int64_t)resident * p->cols;
+    if (fit < std::min<int64_t>(round, ncol)) return false;
+    p->launch = (int)std::min<int64_t>(ncol, std::max<int64_t>(fit / round, 1) * round);
+    p->work += p->work_col * p->launch;
+    return true;
+}
+
 // Of the cluster sizes and widths that fit, the one with the least estimated
 // time for all columns: as many rounds of clusters as are not resident at once,
-// or the SMs' total work where that is more.  K: a filter's order.
+// or the SMs' total work where that is more.  K: a filter's order, a KPM run's steps.
 template <typename T>
 bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
     const double sms = op->h->num_sms;
@@ -1010,6 +1030,7 @@ bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
             const int n = res_resident(p);
             if (n < 1) continue;
             const int groups = res_groups(p, ncol);
+            if (kpm && !kpm_launch(&p, op->dim, (int)sizeof(T), ncol, K, n)) continue;
             double t = std::max((groups + n - 1) / n * p.us, groups * (1 << clog) * p.busy_us / sms);
             const bool rotates = op->kind == OP_QSUN || (p.pinned && !op->h->shared);
             if (rotates && !kpm && K > 0 && groups > n) {
@@ -1150,11 +1171,12 @@ void resident_filter(pf_op *op, cudaStream_t st, const ResPlan &p, void *work, i
 }
 
 template <typename T>
-void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &p, void *work, int M, int R, double a, double b,
+void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &p, void *work, int M, int R, int col0, double a, double b,
                   const T *probes, int64_t ldp, int kind, uint64_t seed, double *part, double *dots) {
     ResArgs<T> r{};
     r.K = M;
     r.X = probes; r.xr = 1; r.xc = ldp;
+    r.col0 = col0;
     r.inva = (T)(1.0 / a);
     r.boa = (T)(b * (1.0 / a));
     r.probe_kind = kind;
@@ -1172,7 +1194,7 @@ void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &p, void *work, int 
     template void resident_prepare<T>(pf_op *, cudaStream_t, const ResPlan &, void *);                             \
     template void resident_filter<T>(pf_op *, cudaStream_t, const ResPlan &, void *, int, int, const double *,     \
                                      double, double, const T *, int64_t, int64_t, T *, int64_t, int64_t);         \
-    template void resident_kpm<T>(pf_op *, cudaStream_t, const ResPlan &, void *, int, int, double, double,        \
+    template void resident_kpm<T>(pf_op *, cudaStream_t, const ResPlan &, void *, int, int, int, double, double,   \
                                   const T *, int64_t, int, uint64_t, double *, double *);
 PF_RES_INST(double)
 PF_RES_INST(float)

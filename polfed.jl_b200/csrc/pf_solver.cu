@@ -305,6 +305,59 @@ struct Filter {
 };
 
 // ------------------------------------------------------------- the KPM
+// The moments by one on-chip recurrence per probe, plan.launch probes at a time,
+// their sums read back kResKpmSums bytes at a time.  false, mu untouched: no
+// column fits a cluster, the step kernels are estimated faster, or the
+// workspace does not fit the device now.
+template <typename T>
+static bool kpm_on_chip(pf_op *op, double a, double b, int N, int R, const T *probes_cm, int64_t ldp, int kind,
+                        uint64_t seed, std::vector<double> &mu) {
+    pf_handle *h = op->h;
+    cudaStream_t st = h->stream;
+    const int M = (N - 1 + 1) / 2;
+    ResPlan plan;
+    if ((int64_t)(M + 1) * R > ((int64_t)1 << 22) || !resident_plan<T>(op, R, true, M, &plan)) return false;
+    const size_t sums = (size_t)2 * (M + 1);   // of a probe
+    const int some = std::max(1, (int)(kResKpmSums / (sums * sizeof(double)) / plan.launch)) * plan.launch;
+    DevArray<unsigned char> work;
+    DevArray<double> parts, rd;
+    try {
+        work.alloc(plan.work);
+        parts.alloc((sums * plan.launch) << plan.clog);
+        rd.alloc(sums * std::min(R, some));
+    } catch (const Error &e) {
+        if (e.code != PF_ERR_NOMEM) throw;
+        cudaGetLastError();
+        return false;
+    }
+    std::vector<double> hr(rd.n);
+    resident_prepare<T>(op, st, plan, work.p);
+    for (int r0 = 0; r0 < R; r0 += some) {
+        const int r1 = std::min(R, r0 + some);
+        for (int c0 = r0; c0 < r1; c0 += plan.launch)
+            resident_kpm<T>(op, st, plan, work.p, M, std::min(plan.launch, r1 - c0), c0, a, b,
+                            probes_cm ? probes_cm + (size_t)c0 * ldp : nullptr, ldp, kind, seed, parts.p,
+                            rd.p + sums * (c0 - r0));
+        PF_CUDA(cudaMemcpyAsync(hr.data(), rd.p, sums * (r1 - r0) * sizeof(double), cudaMemcpyDeviceToHost, st));
+        sync(h);
+        for (int c = r0; c < r1; ++c) {
+            const int c0 = c - (c - r0) % plan.launch, nc = std::min(plan.launch, r1 - c0);
+            const double *v = hr.data() + sums * (c0 - r0) + (c - c0);   // value i of this probe: v[i * nc]
+            const double m0 = v[0];
+            mu[0] += m0;
+            if (M < 1) continue;
+            const double m1 = v[(size_t)3 * nc];   // <v1, v0>
+            if (N > 1) mu[1] += m1;
+            for (int n = 0; n < M; ++n) {
+                if (2 * n + 2 < N) mu[2 * n + 2] += 2.0 * v[(size_t)2 * (n + 1) * nc] - m0;
+                if (n >= 1 && 2 * n + 1 < N) mu[2 * n + 1] += 2.0 * v[((size_t)2 * (n + 1) + 1) * nc] - m1;
+            }
+        }
+    }
+    for (double &m : mu) m *= (double)op->dim / (double)R;
+    return true;
+}
+
 // mu_n = (D/R) sum_r <r|T_n(Htilde)|r>  (Moments.jl:42-140) evaluated with
 // the doubling identities mu_{2n} = 2<v_n,v_n> - mu_0 and
 // mu_{2n+1} = 2<v_{n+1},v_n> - mu_1 per probe (Weisse et al., Rev. Mod. Phys.
@@ -321,29 +374,7 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
     PF_CHECK(N >= 1 && R >= 1, PF_ERR_INVALID, "KPM needs N >= 1 and R >= 1");
     std::vector<double> mu(N, 0.0);
     const int M = (N - 1 + 1) / 2;  // steps: ceil((N-1)/2)
-    // one on-chip recurrence per probe where a column fits a cluster (its dot
-    // partials, 2^(clog + 4) bytes a probe and step, in at most 1 GB)
-    ResPlan plan;
-    if ((int64_t)(M + 1) * R <= ((int64_t)1 << 22) && resident_plan<T>(op, R, true, M, &plan)) {
-        DevArray<unsigned char> work(plan.work);
-        DevArray<double> parts((size_t)2 * (M + 1) * R << plan.clog), rd((size_t)2 * (M + 1) * R);
-        std::vector<double> hr((size_t)2 * (M + 1) * R);
-        resident_prepare<T>(op, st, plan, work.p);
-        resident_kpm<T>(op, st, plan, work.p, M, R, a, b, probes_cm, ldp, kind, seed, parts.p, rd.p);
-        PF_CUDA(cudaMemcpyAsync(hr.data(), rd.p, hr.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-        sync(h);
-        for (int c = 0; c < R; ++c) {
-            const double m0 = hr[c];
-            mu[0] += m0;
-            if (M < 1) continue;
-            const double m1 = hr[(size_t)3 * R + c];   // <v1, v0>
-            if (N > 1) mu[1] += m1;
-            for (int n = 0; n < M; ++n) {
-                if (2 * n + 2 < N) mu[2 * n + 2] += 2.0 * hr[(size_t)2 * (n + 1) * R + c] - m0;
-                if (n >= 1 && 2 * n + 1 < N) mu[2 * n + 1] += 2.0 * hr[((size_t)2 * (n + 1) + 1) * R + c] - m1;
-            }
-        }
-        for (double &m : mu) m *= (double)D / (double)R;
+    if (kpm_on_chip<T>(op, a, b, N, R, probes_cm, ldp, kind, seed, mu)) {
         if (block_matvecs) *block_matvecs += (int64_t)R * M;
         return mu;
     }

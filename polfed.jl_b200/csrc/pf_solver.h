@@ -105,11 +105,17 @@ struct ResPlan {
     int slots = 0;        // groups of columns per launch (0: all in one)
     size_t smem = 0;
     size_t work = 0;      // bytes of device workspace
+    size_t work_col = 0;  // of them, of one column's exchange blocks
+    int launch = 0;       // KPM: columns per launch
     double us = 0, busy_us = 0;   // estimated time of a step of one cluster, and of that the time its SMs are busy
     const void *kern = nullptr;
 };
-// The plan for ncol columns of the operator (K: a filter's order); false: none
-// (a column does not fit a cluster, or the step kernels are estimated faster).
+// Bytes of workspace and dot partials that a KPM run on chip may take even where
+// the step kernels' two blocks of 64 columns are less, and of the sums it reads back at once.
+constexpr size_t kResKpmBytes = size_t(512) << 20, kResKpmSums = size_t(16) << 20;
+// The plan for ncol columns of the operator (K: a filter's order, a KPM run's
+// steps); false: none (a column does not fit a cluster, or the step kernels are
+// estimated faster).
 template <typename T>
 bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *plan);
 // Fills the workspace (plan.work bytes) for the operator; once per workspace.
@@ -120,12 +126,13 @@ void resident_prepare(pf_op *op, cudaStream_t st, const ResPlan &plan, void *wor
 template <typename T>
 void resident_filter(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work, int s, int K, const double *coef,
                      double a, double b, const T *X, int64_t xr, int64_t xc, T *Y, int64_t yr, int64_t yc);
-// M doubling steps from R probes (column-major, or drawn and normalised from
-// the seed when null): dots[0 * R + c] = <v_0, v_0>, and for step n = 1..M
-// dots[2 n * R + c] = <v_n, v_n>, dots[(2 n + 1) * R + c] = <v_n, v_{n-1}>.
+// M doubling steps from R <= plan.launch probes (column-major, or drawn and
+// normalised from the seed as its columns col0 .. when null): dots[0 * R + c] =
+// <v_0, v_0>, and for step n = 1..M dots[2 n * R + c] = <v_n, v_n>,
+// dots[(2 n + 1) * R + c] = <v_n, v_{n-1}>.
 // part: 2 (M + 1) R 2^clog doubles; dots: 2 (M + 1) R.
 template <typename T>
-void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work, int M, int R, double a, double b,
+void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work, int M, int R, int col0, double a, double b,
                   const T *probes, int64_t ldp, int kind, uint64_t seed, double *part, double *dots);
 
 // filter engine (pf_engine.cu): one step launch for every filter in flight

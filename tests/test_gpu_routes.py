@@ -17,7 +17,7 @@ def kernels(torch, call):
     from torch.profiler import ProfilerActivity, profile
     call()
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
         call()
         torch.cuda.synchronize()
     names = {e.name for e in prof.events()}
@@ -65,3 +65,47 @@ def _chain(pkg, L, Lup, seed, distance=1):
     rng = np.random.default_rng(seed)
     bonds = pkg.chain_bonds(L, 1) + (pkg.chain_bonds(L, 2) if distance == 2 else [])
     return pkg.SpinChainOperator(L, Lup, bonds, rng.random(len(bonds)) + 0.5, rng.random(len(bonds)), 2 * rng.random(L) - 1)
+
+
+# ------------------------------------------------------------ moments on chip
+
+def _signs(seed, D, cols):
+    """The +-1 probes of a seed: the low bit of two chained splitmix64 finalisers of (row, column)."""
+    def mix(z):
+        with np.errstate(over="ignore"):
+            z = z + np.uint64(0x9E3779B97F4A7C15)
+            z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+            z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+            return z ^ (z >> np.uint64(31))
+    key = (np.arange(cols, dtype=np.uint64)[:, None] << np.uint64(32)) ^ np.arange(D, dtype=np.uint64)[None, :]
+    return np.where(mix(np.uint64(seed) ^ mix(key)) & np.uint64(1), 1.0, -1.0)
+
+
+@pytest.mark.parametrize("R", [1, 64, 301])
+@pytest.mark.parametrize("kind", ["qsun", "chain"])
+def test_moments_of_many_probes(pkg, cuda, kind, R):
+    """Drawn probes against the same probes given, and against the average of
+    two halves: the columns that one launch takes do not show.  Sums of D
+    products in the same order differ at most in the probes' normalisation, a
+    few eps of each moment's bound |v|^2 = 1 (times 2 for the doubling)."""
+    torch = cuda
+    op = _qsun(pkg, 13, 3, 7) if kind == "qsun" else _chain(pkg, 14, 7, 5)
+    D, N, seed = op.dim, 9, 77
+    P = torch.from_numpy(_signs(seed, D, R)).cuda().t() / math.sqrt(D)
+    drawn = pkg.kpm_moments(op, N, R, 12.0, 0.2, probe_kind="rademacher", seed=seed) / D
+    given = pkg.kpm_moments(op, N, R, 12.0, 0.2, probes=P.t().contiguous().t()) / D
+    assert np.max(np.abs(drawn - given)) < 1e-13
+    if R > 1:
+        h = R // 2
+        part = [pkg.kpm_moments(op, N, n, 12.0, 0.2, probes=P[:, a:a + n].t().contiguous().t()) / D
+                for a, n in ((0, h), (h, R - h))]
+        assert np.max(np.abs(drawn - (h * part[0] + (R - h) * part[1]) / R)) < 1e-13
+
+
+def test_moments_on_chip_hold_a_bounded_workspace(pkg, cuda):
+    """512 MB, however many probes there are."""
+    op = _qsun(pkg, 13, 3, 7)
+    for R in (64, 2000):
+        with PoolHigh() as high:
+            pkg.kpm_moments(op, 3, R, 12.0, 0.2, seed=3)
+        assert high.bytes <= (513 << 20), (R, high.bytes)
