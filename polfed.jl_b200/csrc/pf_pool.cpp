@@ -97,7 +97,13 @@ double solve_footprint(const pf_op *op, const pf_params *p, int s, int nev) {
     const double w = p->precision == PF_PREC_FP64 ? 8.0 : 4.0;
     double bytes = 8.0 * D * std::max(ext + 3.0, maxdim + 3.0 * s);  // Krylov basis + Lanczos blocks
     bytes += 4.0 * D * s * w + 2.0 * 8.0 * D * s;                     // filter blocks, x0 copies
-    bytes += 2.0 * D * 64 * w;                                        // KPM probe blocks
+    double kpm = 2.0 * D * 64 * w;                                    // KPM probe blocks of the step kernels
+    if (D <= 262144.0) {   // or those of a run on chip (kpm_launch), where a column may fit a cluster
+        const double M = std::max(p->dos_N / 2, 0) + 1.0, R = std::max(p->dos_R, 0);
+        kpm = std::max(kpm, std::min((double)kResKpmBytes, R * (2.0 * D * w + 256.0 * M)) +
+                                std::min((double)kResKpmSums, 16.0 * M * R));
+    }
+    bytes += kpm;
     bytes += 2.0 * 8.0 * D * nev;                                     // Ritz vectors and H psi
     bytes += 3.0 * 8.0 * maxdim * maxdim + (64 << 20);                // projected matrix, its eigenvectors, slack
     bytes += (double)chain_list_bytes(op);                            // a chain's flip list

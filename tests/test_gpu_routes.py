@@ -109,3 +109,14 @@ def test_moments_on_chip_hold_a_bounded_workspace(pkg, cuda):
         with PoolHigh() as high:
             pkg.kpm_moments(op, 3, R, 12.0, 0.2, seed=3)
         assert high.bytes <= (513 << 20), (R, high.bytes)
+
+
+def test_solve_stays_within_the_footprint_a_pool_charges(pkg, cuda):
+    """A request of few pairs and many probes, whose moments hold the most."""
+    op = _qsun(pkg, 13, 3, 7)
+    x0 = np.random.default_rng(1).standard_normal((op.dim, 1))
+    kw = dict(mapping=pkg.MappingConfig(Emin=-12.0, Emax=12.0), transform=pkg.TransformConfig(order=12),
+              dos=pkg.DoSConfig(N=60, R=1200, seed=3))
+    with PoolHigh() as high:
+        pkg.polfed(op, x0, 1, ("rescaled", 0.1), vecs=False, **kw)
+    assert high.bytes <= pkg.SolverPool.footprint(op, 1, ("rescaled", 0.1), 1, **kw), high.bytes
