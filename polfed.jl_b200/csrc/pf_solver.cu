@@ -129,20 +129,32 @@ static void sync(pf_handle *h) { PF_CUDA(cudaStreamSynchronize(h->stream)); }
 // it lives; empty for other operators and where it would take more than a
 // sixteenth of the device's memory (or does not fit): the steps then rank their
 // flips themselves.
-static size_t device_bytes(int device) {
-    thread_local std::map<int, size_t> known;
-    auto it = known.find(device);
-    if (it != known.end()) return it->second;
+static void device_bytes(int device, double *total, double *available) {
     size_t free_b = 0, total_b = 0;
+    cudaMemPool_t pool;
+    uint64_t held = 0, used = 0;
     PF_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    return known[device] = total_b;
+    PF_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
+    PF_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+    PF_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    *total = (double)total_b;
+    *available = (double)free_b + (double)(held - std::min(held, used));
 }
+// Lists of at most this many bytes are made without asking for the device's
+// memory (two driver calls): a solve's footprint has more slack than that.
+constexpr size_t kSmallList = size_t(32) << 20;
 struct ChainList {
     DevArray<unsigned char> mem;
     const void *get() const { return mem.p; }
-    void make(pf_op *op, cudaStream_t st) {
+    // rest: bytes that the call allocates after the list, which must still fit
+    void make(pf_op *op, cudaStream_t st, double rest) {
         const size_t bytes = chain_list_bytes(op);
-        if (bytes == 0 || mem.p || bytes > device_bytes(op->h->device) / 16) return;
+        if (bytes == 0 || mem.p) return;
+        if (bytes > kSmallList) {
+            double total, available;
+            device_bytes(op->h->device, &total, &available);
+            if ((double)bytes > total / 16 || (double)bytes + rest > available) return;
+        }
         try {
             mem.alloc(bytes);
         } catch (const Error &e) {
@@ -152,6 +164,12 @@ struct ChainList {
         }
         build_chain_list(op, st, mem.p);
     }
+};
+// The list of the call that a step, filter or probe belongs to: null with own =
+// false where that call decided to hold none.
+struct ListRef {
+    const void *list = nullptr;
+    bool own = true;   // no such call: it may make its own
 };
 // Steps from which a call makes its own list: making it takes about as long as
 // one step with it, and a step with it two thirds of one without.
@@ -185,16 +203,16 @@ struct Filter {
     DevArray<unsigned char> work;
     DevArray<double> dc;
     ChainList own_list;   // of a chain, unless the caller has one
-    const void *list;
+    const void *list = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 
     // io = false: only the two work blocks (the filter engine reads and
     // writes the caller's blocks directly)
     Filter(pf_op *op_, int s_, const std::vector<double> &coeffs, double a_, double b_, bool io = true,
-           const void *list_ = nullptr)
+           ListRef lr = {})
         : op(op_), s(s_), K((int)coeffs.size() - 1), c(coeffs), a(a_), b(b_),
-          resident(io && resident_filter_plan<T>(op_, s_, (int)coeffs.size() - 1, &plan)), list(nullptr) {
+          resident(io && resident_filter_plan<T>(op_, s_, (int)coeffs.size() - 1, &plan)) {
         const size_t n = (size_t)op->dim * s;
         if (resident) {
             dc.alloc(c.size());
@@ -210,9 +228,9 @@ struct Filter {
         if (K >= 1) A.alloc(n);
         if (K >= 2) B.alloc(n);
         if (io && op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T))) {
-            list = list_;
-            if (!list && K >= kListSteps) {
-                own_list.make(op, op->h->stream);
+            list = lr.list;
+            if (lr.own && K >= kListSteps) {
+                own_list.make(op, op->h->stream, 0.0);
                 list = own_list.get();
             }
         }
@@ -367,7 +385,7 @@ static bool kpm_on_chip(pf_op *op, double a, double b, int N, int R, const T *pr
 template <typename T>
 static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int R, const T *probes_cm,
                                        int64_t ldp, int kind, uint64_t seed, int64_t *block_matvecs,
-                                       const void *list = nullptr) {
+                                       ListRef lr = {}) {
     pf_handle *h = op->h;
     const int64_t D = op->dim;
     cudaStream_t st = h->stream;
@@ -383,8 +401,9 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
     DevArray<double> dots((size_t)std::max(M, 1) * 2 * RB), n0(RB), scl(RB);
     std::vector<double> hd((size_t)std::max(M, 1) * 2 * RB), h0(RB), hs(RB);
     ChainList own_list;
-    if (!list && (int64_t)M * ((R + 63) / 64) >= kListSteps) {
-        own_list.make(op, st);
+    const void *list = lr.list;
+    if (lr.own && (int64_t)M * ((R + 63) / 64) >= kListSteps) {
+        own_list.make(op, st, 0.0);
         list = own_list.get();
     }
     auto step = [&](int nb, const T *q, const T *p, T *out, double alpha, double beta, int flags, double *dst) {
@@ -1373,7 +1392,7 @@ static void cholqr2_block(pf_handle *h, double *W, int64_t D, int m) {
 // Returns the number of passes run.
 static int refine_fp64(pf_op *op, const std::vector<double> &coeffs, double a, double b, int nev, double eigentol,
                        int max_passes, DevArray<double> &Psi, int m, std::vector<double> &vals,
-                       std::vector<double> &resid, const void *list) {
+                       std::vector<double> &resid, ListRef lr) {
     pf_handle *h = op->h;
     cudaStream_t st = h->stream;
     const int64_t D = op->dim;
@@ -1398,7 +1417,7 @@ static int refine_fp64(pf_op *op, const std::vector<double> &coeffs, double a, d
         for (int c0 = 0; c0 < m; c0 += wmax) {
             const int wc = std::min(wmax, m - c0);
             auto &f = filters[wc];
-            if (!f) f.reset(new Filter<double>(op, wc, coeffs, a, b, true, list));
+            if (!f) f.reset(new Filter<double>(op, wc, coeffs, a, b, true, lr));
             if (f->resident) {
                 f->run_resident(st, Psi.p + c0, m, 1, W.p + c0, m, 1);
                 continue;
@@ -1473,13 +1492,17 @@ static pf_handle *aux_handle(pf_handle *h) {
     return h->aux;
 }
 
+// Device bytes of the two probes' Lanczos runs, their bases and a few vectors each.
+static double probe_bytes(int64_t D, int maxdim) { return 2.0 * 8.0 * (double)D * (std::min<double>(maxdim, (double)D) + 8.0); }
+
 static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, double tol, double eigentol, double *Emin,
                                 double *Emax, int *qr_restarts = nullptr, bool host_qr = false,
-                                const void *list = nullptr) {
+                                ListRef lr = {}) {
     const int64_t D = op->dim;
     ChainList own_list;
-    if (!list) {
-        own_list.make(op, op->h->stream);
+    const void *list = lr.list;
+    if (lr.own) {
+        own_list.make(op, op->h->stream, probe_bytes(D, maxdim));
         list = own_list.get();
     }
     // The :SR probe runs here and the :LR probe at the same time on the
@@ -1795,10 +1818,12 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     }
 
     // a chain's flips are listed once for the whole solve (its probes, its
-    // moments and its filter), unless the solve itself is near the device's memory
+    // moments and its filter), if the rest of the solve still fits beside the list
     ChainList chain_list;
-    if (solve_footprint(op, P, s, nev) < 0.85 * (double)device_bytes(h->device)) chain_list.make(op, st);
-    const void *list = chain_list.get();
+    const int probe_dim = P->extrema_maxdim > 0 ? P->extrema_maxdim : 1000;
+    chain_list.make(op, st, solve_footprint(op, P, s, nev) - (double)chain_list_bytes(op) +
+                                (P->has_Emin && P->has_Emax ? 0.0 : probe_bytes(D, probe_dim) / 2));
+    const ListRef list{chain_list.get(), false};
 
     // mapping plan (Plan.jl:128-191)
     double Emin = P->Emin, Emax = P->Emax;
@@ -1807,7 +1832,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
         if (!P->has_Emin || !P->has_Emax) {
             double lo = 0, hi = 0;
             // v0 = x0[:, 1] (column 0 of the column-major copy)
-            extrema_from_device(op, xcm.p, P->extrema_maxdim > 0 ? P->extrema_maxdim : 1000, 1e-14, 1e-8, &lo, &hi,
+            extrema_from_device(op, xcm.p, probe_dim, 1e-14, 1e-8, &lo, &hi,
                                 &R.qr_restarts, P->host_qr != 0, list);
             if (!P->has_Emin) Emin = lo;
             if (!P->has_Emax) Emax = hi;
@@ -1887,7 +1912,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     ResPlan onchip;
     const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, (int)coeffs.size() - 1, &onchip)
                                                  : resident_filter_plan<float>(op, s, (int)coeffs.size() - 1, &onchip));
-    if (P->autotune && steps && (eng || !list || op->slab_cols > 0)) {
+    if (P->autotune && steps && (eng || !list.list || op->slab_cols > 0)) {
         bool have;
         {
             std::lock_guard<std::mutex> lock(op->tune_mu);

@@ -120,3 +120,44 @@ def test_solve_stays_within_the_footprint_a_pool_charges(pkg, cuda):
     with PoolHigh() as high:
         pkg.polfed(op, x0, 1, ("rescaled", 0.1), vecs=False, **kw)
     assert high.bytes <= pkg.SolverPool.footprint(op, 1, ("rescaled", 0.1), 1, **kw), high.bytes
+
+
+# ------------------------------------------------------------ a solve's flip list
+
+_NEAR_FULL = """
+import ctypes, sys
+import numpy as np, torch
+sys.path.insert(0, {root!r})
+import __graft_entry__ as ge
+pkg = ge.load_package()
+rng = np.random.default_rng(1)
+L = 24
+bonds = pkg.chain_bonds(L, 1)
+op = pkg.SpinChainOperator(L, L // 2, bonds, [1.0] * L, [1.0] * L, 2 * rng.random(L) - 1)
+x0 = rng.standard_normal((op.dim, 1))
+solve = lambda: pkg.polfed(op, x0, 1, ("rescaled", 0.1), vecs=False, mapping=pkg.MappingConfig(Emin=-30.0, Emax=30.0),
+                           transform=pkg.TransformConfig(order=9), dos=pkg.DoSConfig(N=4, R=1, seed=3))
+cu, pool, v = ctypes.CDLL("libcuda.so.1"), ctypes.c_void_p(), ctypes.c_uint64(0)
+solve()
+torch.cuda.synchronize()
+assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+assert cu.cuMemPoolGetAttribute(pool, 8, ctypes.byref(v)) == 0      # the solve's high-water mark, with the list
+assert cu.cuMemPoolTrimTo(pool, ctypes.c_size_t(0)) == 0
+listed = op.dim * (L // 4 + 1) * 16
+free = torch.cuda.mem_get_info()[0]
+keep = torch.empty(int(free - (v.value - listed // 2)), dtype=torch.uint8, device="cuda")
+solve()
+print("solved", v.value, listed)
+"""
+
+
+def test_solve_without_room_for_a_flip_list(pkg, cuda):
+    """A solve whose flip list (303 MB) would leave too little for its basis runs
+    without one.  In a process of its own, which leaves the solve half a list
+    less than it took with the list."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _NEAR_FULL.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.startswith("solved"), r.stdout + r.stderr
