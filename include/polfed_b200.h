@@ -246,7 +246,8 @@ int pf_step_variant(pf_op *op, int dtype, int s, int *width, int *gather_batch, 
  * pf_set_step_variant (for instance in another process). */
 int pf_step_profile(pf_op *op, int dtype, int s, int *profile);
 /* Pin the step-kernel variant for (dtype, s) without timing (a width the
- * autotuner could have chosen); later launches on this operator use it. */
+ * autotuner could have chosen); later applies, recurrences, final sums, filters
+ * and (s = 1, FP64) extremal probes of this operator run that step. */
 int pf_set_step_width(pf_op *op, int dtype, int s, int width);
 /* Same with a profile: 0 = the width's default gather batch and register cap,
  * 1..4 = (8 gathers, 2 CTAs/SM), (8, 3), (4, 4), (8, 4); 5 = Quantum Sun

@@ -193,7 +193,7 @@ struct pf_op {
     // autotuned columns-per-thread of the step kernel, keyed by (element bytes, s)
     std::mutex tune_mu;
     std::map<std::pair<int, int>, int> tuned_width;
-    // the (element bytes, s) whose variant the caller pinned: their filters run step by step
+    // the (element bytes, s) whose variant the caller pinned: their steps run that variant, their filters step by step
     std::set<std::pair<int, int>> pinned_width;
     // host copies of the defining parameters (for reports and re-creation)
     std::vector<int32_t> bonds;
@@ -271,6 +271,8 @@ double gather_peak(pf_handle *h, int log2_rows);
 // Take the variant for (s, dtype) from the persistent tuning cache, if it holds
 // one for this device, model and size; returns whether it did.
 bool cached_step_variant(pf_op *op, int s, int dtype);
+// Whether the caller pinned the step of s columns: the forms that replace it are not offered then.
+bool pinned_step(pf_op *op, int s, int elem);
 // (gather batch U, resident CTAs per SM) of a variant code for element size elem.
 void variant_params(int code, int elem, int *V, int *U, int *MB);
 

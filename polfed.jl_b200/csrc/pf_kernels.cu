@@ -910,6 +910,11 @@ void launch_step_width(pf_op *op, cudaStream_t st, int64_t D, int s, const T *q,
     }
 }
 
+bool pinned_step(pf_op *op, int s, int elem) {
+    std::lock_guard<std::mutex> lock(op->tune_mu);
+    return op->pinned_width.count(std::make_pair(elem, s)) > 0;
+}
+
 template <typename T>
 void launch_step(pf_op *op, cudaStream_t st, int64_t D, int s, const T *q, const T *p,
                  const T *x, T *out, double cx, double alpha, double beta, double inva,

@@ -424,7 +424,9 @@ static void op_step_cm(pf_op *op, int s, const T *q, const T *p, const T *x, T *
         launch_step<T>(op, h->stream, D, 1, q, p, x, out, cx, alpha, beta, 1.0 / a, b, flags, nullptr);
         return;
     }
-    if (launch_step_cm<T>(op, h->stream, s, q, p, x, out, ld, ldout, cx, alpha, beta, 1.0 / a, b)) return;
+    if (!pinned_step(op, s, (int)sizeof(T)) &&
+        launch_step_cm<T>(op, h->stream, s, q, p, x, out, ld, ldout, cx, alpha, beta, 1.0 / a, b))
+        return;
     const size_t n = (size_t)D * s;
     T *base = (T *)handle_scratch(h, 4 * n * sizeof(T));
     T *qr = base, *pr = base + n, *xr = base + 2 * n, *outr = base + 3 * n;

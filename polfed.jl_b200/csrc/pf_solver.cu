@@ -179,10 +179,6 @@ constexpr int kListSteps = 8;
 // Whether an s-column filter runs whole on chip: it fits and is estimated
 // faster than the step kernels, and the caller asked for neither column slabs
 // nor a step variant of their own.
-static bool pinned_step(pf_op *op, int s, int elem) {
-    std::lock_guard<std::mutex> lock(op->tune_mu);
-    return op->pinned_width.count(std::make_pair(elem, s)) > 0;
-}
 template <typename T>
 static bool resident_filter_plan(pf_op *op, int s, int K, ResPlan *plan) {
     return op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T)) && resident_plan<T>(op, s, false, K, plan);
@@ -1501,7 +1497,9 @@ static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, dou
     const int64_t D = op->dim;
     ChainList own_list;
     const void *list = lr.list;
-    if (lr.own) {
+    if (pinned_step(op, 1, (int)sizeof(double))) {
+        list = nullptr;   // the step the caller chose
+    } else if (lr.own) {
         own_list.make(op, op->h->stream, probe_bytes(D, maxdim));
         list = own_list.get();
     }

@@ -161,3 +161,32 @@ def test_solve_without_room_for_a_flip_list(pkg, cuda):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _NEAR_FULL.format(root=root)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.startswith("solved"), r.stdout + r.stderr
+
+
+# ------------------------------------------------------------ pinned variants
+
+@pytest.mark.parametrize("kind", ["qsun", "chain"])
+def test_pinned_variant_governs_every_later_step(pkg, cuda, kind):
+    """Applies, recurrences, final sums, filters and extremal probes of a width
+    run the step kernel that the caller pinned for it; results are the same bits."""
+    torch = cuda
+    mk = (lambda: _qsun(pkg, 8, 3, 2)) if kind == "qsun" else (lambda: _chain(pkg, 12, 6, 3))
+    op, ref, s = mk(), mk(), 4
+    pkg.set_step_width(op, s, 2)
+    pkg.set_step_width(op, 1, 1)
+    q, p, x, y, z = (_block(torch, op.dim, s, torch.float64, k) for k in range(5))
+    v0 = np.random.default_rng(1).standard_normal(op.dim)
+    calls = {"apply": lambda o, out: pkg.apply(o, out, q, 3.0, 0.2),
+             "recurrence": lambda o, out: pkg.clenshaw_recurrence(o, out, q, p, 0.7, x, 3.0, 0.2),
+             "finalsum": lambda o, out: pkg.clenshaw_finalsum(o, q, p, 0.7, out, x, 3.0, 0.2),
+             "filter": lambda o, out: pkg.chebyshev_filter(o, out, q, np.cos(np.arange(20)), 9.0, 0.1)}
+    for name, call in calls.items():
+        names = kernels(torch, lambda: call(op, y))
+        assert ran(names, "k_step"), (name, names)
+        for other in ("k_step_cm", "k_res_qsun", "k_res_list", "k_res_pinned", "k_step_chain_list"):
+            assert not ran(names, other), (name, other)
+        call(ref, z)
+        assert torch.equal(y, z), name
+    names = kernels(torch, lambda: pkg.lanczos_extrema(op, v0))
+    assert ran(names, "k_step") and not ran(names, "k_step_chain_list"), names
+    assert pkg.lanczos_extrema(op, v0) == pkg.lanczos_extrema(ref, v0)
