@@ -218,7 +218,9 @@ int pf_kpm_moments(pf_op *op, int dtype, double a, double b, int N, int R,
  * 8, 16 and PF_WIDTH_COOP (0 where not offered).  Every variant computes the
  * same sums in the same order.  The choice is also written to a persistent
  * cache ($POLFED_B200_TUNE_CACHE, else ~/.cache/polfed_b200/step_variants.json)
- * that pf_solve consults before timing. */
+ * that pf_solve consults before timing.  A variant pinned for (dtype, s) before
+ * is released.  The choice serves what runs step by step: filters that run on
+ * chip or from a chain's flip list do not use it. */
 #define PF_WIDTH_COOP 0
 int pf_autotune(pf_op *op, int dtype, int s, int *width, float *times_ms);
 /* G = B^T r on the 5th-generation tensor cores (tcgen05.mma, BF16 inputs,
@@ -247,7 +249,8 @@ int pf_step_variant(pf_op *op, int dtype, int s, int *width, int *gather_batch, 
 int pf_step_profile(pf_op *op, int dtype, int s, int *profile);
 /* Pin the step-kernel variant for (dtype, s) without timing (a width the
  * autotuner could have chosen); later applies, recurrences, final sums, filters
- * and (s = 1, FP64) extremal probes of this operator run that step. */
+ * and (s = 1, FP64) extremal probes of this operator run that step, until
+ * pf_autotune chooses one for (dtype, s). */
 int pf_set_step_width(pf_op *op, int dtype, int s, int width);
 /* Same with a profile: 0 = the width's default gather batch and register cap,
  * 1..4 = (8 gathers, 2 CTAs/SM), (8, 3), (4, 4), (8, 4); 5 = Quantum Sun

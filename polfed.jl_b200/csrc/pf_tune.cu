@@ -185,6 +185,7 @@ static int tune_typed(pf_op *op, int s, std::vector<std::pair<int, float>> *timi
     {
         std::lock_guard<std::mutex> lock(op->tune_mu);
         op->tuned_width[std::make_pair((int)sizeof(T), s)] = best;
+        op->pinned_width.erase(std::make_pair((int)sizeof(T), s));
     }
     {
         std::lock_guard<std::mutex> lock(g_cache_mu);

@@ -190,3 +190,17 @@ def test_pinned_variant_governs_every_later_step(pkg, cuda, kind):
     names = kernels(torch, lambda: pkg.lanczos_extrema(op, v0))
     assert ran(names, "k_step") and not ran(names, "k_step_chain_list"), names
     assert pkg.lanczos_extrema(op, v0) == pkg.lanczos_extrema(ref, v0)
+
+
+def test_autotune_releases_a_pinned_variant(pkg, cuda):
+    """A pin holds until the caller has the variant chosen by timing again."""
+    torch = cuda
+    op, s = _chain(pkg, 12, 6, 3), 4
+    X = _block(torch, op.dim, s, torch.float64, 1)
+    Y = torch.empty_like(X)
+    call = lambda: pkg.chebyshev_filter(op, Y, X, np.cos(np.arange(20)), 9.0, 0.1)
+    pkg.set_step_width(op, s, 2)
+    assert ran(kernels(torch, call), "k_step")
+    pkg.autotune(op, s)
+    names = kernels(torch, call)
+    assert ran(names, "k_res_pinned") and not ran(names, "k_step"), names
