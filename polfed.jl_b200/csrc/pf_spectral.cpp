@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <queue>
 #include <stdexcept>
 
@@ -287,6 +288,67 @@ std::vector<double> normalized_coefficients(const TransformState &t) {
     const double norm_ = 1.0 / cheb_clenshaw(c.data(), t.order, t.target) * t.normalization;
     for (double &v : c) v *= norm_;
     return c;
+}
+
+bool tridiag_vector(const std::vector<double> &d, const std::vector<double> &e, double lam,
+                           std::vector<double> &z) {
+    const int n = (int)d.size();
+    double nrm = 0.0;
+    for (int i = 0; i < n; ++i)
+        nrm = std::max(nrm, std::fabs(d[i]) + (i > 0 ? std::fabs(e[i - 1]) : 0.0) + (i + 1 < n ? std::fabs(e[i]) : 0.0));
+    if (!(nrm > 0.0) || !std::isfinite(nrm) || !std::isfinite(lam)) return false;
+    const double tiny = std::numeric_limits<double>::epsilon() * nrm;
+    // the factors: rows of U (three diagonals), the multipliers and the exchanges
+    std::vector<double> u0(n), u1(n, 0.0), u2(n, 0.0), l(n, 0.0);
+    std::vector<char> swapped(n, 0);
+    double p0 = d[0] - lam, p1 = n > 1 ? e[0] : 0.0, p2 = 0.0;
+    for (int i = 0; i + 1 < n; ++i) {
+        const double q0 = e[i], q1 = d[i + 1] - lam, q2 = i + 2 < n ? e[i + 1] : 0.0;
+        if (std::fabs(q0) > std::fabs(p0)) {
+            swapped[i] = 1;
+            l[i] = p0 / q0;
+            u0[i] = q0, u1[i] = q1, u2[i] = q2;
+            p0 = p1 - l[i] * q1, p1 = p2 - l[i] * q2;
+        } else {
+            if (std::fabs(p0) < tiny) p0 = tiny;
+            l[i] = q0 / p0;
+            u0[i] = p0, u1[i] = p1, u2[i] = p2;
+            p0 = q1 - l[i] * p1, p1 = q2 - l[i] * p2;
+        }
+        p2 = 0.0;
+    }
+    u0[n - 1] = std::fabs(p0) < tiny ? tiny : p0;
+    z.assign(n, 1.0 / std::sqrt((double)n));
+    for (int it = 0; it < 3; ++it) {
+        if (it > 0)
+            for (int i = 0; i + 1 < n; ++i) {
+                if (swapped[i]) std::swap(z[i], z[i + 1]);
+                z[i + 1] -= l[i] * z[i];
+            }
+        double s2 = 0.0, big = 0.0;
+        for (int i = n - 1; i >= 0; --i) {
+            double v = z[i];
+            if (i + 1 < n) v -= u1[i] * z[i + 1];
+            if (i + 2 < n) v -= u2[i] * z[i + 2];
+            z[i] = v / u0[i];
+            big = std::max(big, std::fabs(z[i]));
+            if (big > 1e100) {
+                for (int j = i; j < n; ++j) z[j] *= 1e-100;
+                for (int j = 0; j < i; ++j) z[j] *= 1e-100;
+                big *= 1e-100;
+            }
+        }
+        for (double v : z) s2 += v * v;
+        s2 = std::sqrt(s2);
+        if (!(s2 > 0.0) || !std::isfinite(s2)) return false;
+        for (double &v : z) v /= s2;
+    }
+    double r2 = 0.0;
+    for (int i = 0; i < n; ++i) {
+        const double r = (d[i] - lam) * z[i] + (i > 0 ? e[i - 1] * z[i - 1] : 0.0) + (i + 1 < n ? e[i] * z[i + 1] : 0.0);
+        r2 += r * r;
+    }
+    return std::sqrt(r2) <= 64.0 * tiny;
 }
 
 }  // namespace pf

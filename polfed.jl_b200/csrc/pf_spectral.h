@@ -27,6 +27,13 @@ double quadgk(const std::function<void(const double *, double *, int)> &f, doubl
               double rtol, long maxevals);
 double analytical_order(double lam, double delta);
 
+// The unit eigenvector z of the tridiagonal matrix (d, e) for its eigenvalue
+// lam, by inverse iteration (Gaussian elimination with row exchanges, three
+// solves).  Returns false if its residual is above 64 roundings of the matrix's
+// norm (the dense solver's vectors have a few): lam is not an eigenvalue to
+// rounding, or the iteration did not settle.
+bool tridiag_vector(const std::vector<double> &d, const std::vector<double> &e, double lam, std::vector<double> &z);
+
 // TransformPlan of Plan.jl:32-44 in rescaled units.
 struct TransformState {
     int target_kind = 0;
