@@ -30,15 +30,23 @@ constexpr int kThreads = 256;
 
 // Deterministic "last block reduces" epilogue: every block writes its
 // per-column partials, the block that finishes last sums them: each value over
-// a fixed number of strided runs (as many as the block has threads for), a
-// run's loads sixteen in flight, then the runs in order.  The partials are read
+// a number of strided runs fixed by the grid (of sixteen partials or more, and
+// no more than the block has threads for), a run's loads sixteen in flight, then
+// the runs in order.  The partials are read
 // through L2 (__ldcg: other blocks wrote them before the counter told this
 // block it is last).  With one run of eight loads in flight the tail took 20 us
-// for 444 blocks of 128 values.  runs: blockDim.x doubles of shared memory
+// for 444 blocks of 128 values; as many runs as threads, whatever the grid, take
+// longer to sum than to read (steps of 313 blocks, 2 values: 11.2 -> 10.1 us a
+// step; of 1444 blocks, 8 values: 24.8 -> 21.8).  One block has nothing to sum:
+// 6.9 -> 4.2 us a step of 32 rows.  runs: blockDim.x doubles of shared memory
 // that blockvals does not overlap.
 static __device__ void finish_reduction(int nvals, const double *blockvals, double *partials, unsigned int *counter,
                                         double *out, double *runs) {
     __shared__ bool last;
+    if (gridDim.x == 1) {
+        for (int c = threadIdx.x; c < nvals; c += blockDim.x) out[c] = blockvals[c];
+        return;
+    }
     for (int c = threadIdx.x; c < nvals; c += blockDim.x)
         partials[(size_t)blockIdx.x * nvals + c] = blockvals[c];
     __threadfence();
@@ -51,20 +59,18 @@ static __device__ void finish_reduction(int nvals, const double *blockvals, doub
     if (last) {
         __threadfence();
         const unsigned int nb = gridDim.x;
-        const int Q = nvals < (int)blockDim.x ? (int)blockDim.x / nvals : 1;
+        const int Q = max(1, min((int)blockDim.x / nvals, (int)((nb + 15) / 16)));
         for (int w = threadIdx.x; w < Q * nvals; w += blockDim.x) {
             const int c = w % nvals, q = w / nvals;
             double acc = 0.0;
             const double *col = partials + c;
-            unsigned int b = q;
-            for (; b + 15 * Q < nb; b += 16 * Q) {
+            for (unsigned int b = q; b < nb; b += 16 * Q) {
                 double x[16];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) x[u] = __ldcg(col + (size_t)(b + u * Q) * nvals);
+                for (int u = 0; u < 16; ++u) x[u] = b + u * Q < nb ? __ldcg(col + (size_t)(b + u * Q) * nvals) : 0.0;
 #pragma unroll
                 for (int u = 0; u < 16; ++u) acc += x[u];
             }
-            for (; b < nb; b += Q) acc += __ldcg(col + (size_t)b * nvals);
             if (Q == 1) out[c] = acc;
             else runs[w] = acc;
         }
