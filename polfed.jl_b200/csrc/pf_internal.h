@@ -100,6 +100,17 @@ struct CsrDesc {
     const T *values;         // nnz
 };
 
+// What decides how fast a CSR matrix's gathers run.  A slice is 32 consecutive
+// rows; its n-th gather is the n-th entry of each of its rows.
+struct CsrShape {
+    int max_row = 0;           // entries of the longest row
+    double slots = 0;          // row places of all slices, their rows as long as the longest, in eights
+    // of a split of the rows into 2^k equal ranges: entries whose column is not
+    // in their row's range, and the sectors of 32 bytes (four FP64 columns) these
+    // are gathered from, counted per gather
+    double far_entries[5] = {}, far[5] = {};
+};
+
 enum OpKind { OP_CHAIN = 0, OP_QSUN = 1, OP_CSR = 2 };
 
 // Number of entries of the chunked rank table for an L-bit sector:
@@ -171,7 +182,7 @@ struct pf_op {
     pf::CsrDesc<double> csr64{};
     pf::CsrDesc<float> csr32{};
     int64_t nnz = 0;
-    int max_row = 0;                  // CSR: entries of the longest row
+    pf::CsrShape shape;               // CSR: what the estimates of a step need to know
     // > 0: the real embedding [[A, -B], [B, A]] of a complex Hermitian H = A + iB
     // of this dimension (dim = 2 complex_dim); solved by solve_hermitian
     int64_t complex_dim = 0;
@@ -271,6 +282,8 @@ double gather_peak(pf_handle *h, int log2_rows);
 // Take the variant for (s, dtype) from the persistent tuning cache, if it holds
 // one for this device, model and size; returns whether it did.
 bool cached_step_variant(pf_op *op, int s, int dtype);
+// Columns per thread of a step with fused dots on s columns.
+int dots_width(int s, int elem_bytes);
 // Whether the caller pinned the step of s columns: the forms that replace it are not offered then.
 bool pinned_step(pf_op *op, int s, int elem);
 // (gather batch U, resident CTAs per SM) of a variant code for element size elem.

@@ -865,6 +865,13 @@ int default_width(int s, int elem_bytes) {
     return 1;
 }
 
+// The fused dots keep 2V FP64 accumulators per thread: at most 32 bytes of columns.
+int dots_width(int s, int elem_bytes) {
+    int V = default_width(s, elem_bytes);
+    while (V > 1 && (V * elem_bytes > 32 || kThreads % (s / V) != 0)) V /= 2;
+    return V;
+}
+
 template <typename T>
 void launch_step_width(pf_op *op, cudaStream_t st, int64_t D, int s, const T *q, const T *p, const T *x, T *out,
                        double cx, double alpha, double beta, double inva, double shift, int flags, double *dots,
@@ -925,11 +932,7 @@ void launch_step(pf_op *op, cudaStream_t st, int64_t D, int s, const T *q, const
         auto it = op->tuned_width.find(std::make_pair((int)sizeof(T), s));
         if (it != op->tuned_width.end()) V = it->second;
     }
-    if (flags & StepFlags::DOTS) {
-        // the fused dots keep 2V FP64 accumulators per thread: at most 32 bytes of columns
-        V = default_width(s, (int)sizeof(T));
-        while (V > 1 && (V * (int)sizeof(T) > 32 || kThreads % (s / V) != 0)) V /= 2;
-    }
+    if (flags & StepFlags::DOTS) V = dots_width(s, (int)sizeof(T));
     const bool slab = ld > 0 && ld != s;
     if (V == kCoopWidth && (slab || !coop_eligible(op, s, flags))) V = default_width(s, (int)sizeof(T));
     if (variant_profile(V) != 0 && (flags & StepFlags::DOTS)) V = variant_width(V);

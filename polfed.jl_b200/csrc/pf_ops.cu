@@ -296,24 +296,59 @@ pf_op *create_csr_hermitian(pf_handle *h, int64_t D, int64_t nnz, const int64_t 
     return op;
 }
 
-// Entries of the longest row of a CSR matrix on the device.
-static __global__ void k_csr_longest_row(const int64_t *__restrict__ indptr, int64_t D, int *out) {
-    int most = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x)
-        most = max(most, (int)min(indptr[i + 1] - indptr[i], (int64_t)INT32_MAX));
-    if (most > 0) atomicMax(out, most);
+// CsrShape, counted on the device: a warp per slice.  out: max_row, slots / 32,
+// far_entries[1..4], far[1..4].
+static __global__ void k_csr_shape(const int64_t *__restrict__ indptr, const int32_t *__restrict__ indices, int64_t D,
+                                   unsigned long long *out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
+    unsigned long long most = 0, slots = 0, fe[5] = {0, 0, 0, 0, 0}, fs[5] = {0, 0, 0, 0, 0};
+    for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 32; w * 32 < D; w += warps) {
+        const int64_t row = w * 32 + lane;
+        const int64_t p = row < D ? indptr[row] : 0;
+        const unsigned cnt = row < D ? (unsigned)(indptr[row + 1] - p) : 0u;
+        const unsigned longest = __reduce_max_sync(0xffffffffu, cnt);
+        most = max(most, (unsigned long long)longest);
+        slots += (longest + 7u) / 8u * 8u;
+        for (unsigned n = 0; n < longest; ++n) {
+            const uint32_t col = n < cnt ? (uint32_t)indices[p + n] : 0xffffffffu;
+            const unsigned same = __match_any_sync(0xffffffffu, col >> 2);
+#pragma unroll
+            for (int k = 1; k <= 4; ++k) {
+                const uint32_t range = (uint32_t)((D + (1 << k) - 1) >> k);
+                const unsigned away = __ballot_sync(0xffffffffu, n < cnt && col / range != (uint32_t)row / range);
+                fe[k] += __popc(away);
+                fs[k] += __popc(__ballot_sync(0xffffffffu, (away >> lane & 1u) && (same & away) >> lane == 1u));
+            }
+        }
+    }
+    if (lane == 0) {
+        atomicMax(out, most);
+        atomicAdd(out + 1, slots);
+        for (int k = 1; k <= 4; ++k) {
+            atomicAdd(out + 1 + k, fe[k]);
+            atomicAdd(out + 5 + k, fs[k]);
+        }
+    }
 }
 
-static int csr_longest_row(pf_handle *h, int64_t D, const int64_t *indptr) {
-    int *out = static_cast<int *>(handle_scratch(h, sizeof(int)));
-    int most = 0;
-    PF_CUDA(cudaMemsetAsync(out, 0, sizeof(int), h->stream));
-    k_csr_longest_row<<<grid_for(h, D, 256, 8), 256, 0, h->stream>>>(indptr, D, out);
+static CsrShape csr_shape(pf_handle *h, int64_t D, const int64_t *indptr, const int32_t *indices) {
+    unsigned long long v[10] = {};
+    auto *out = static_cast<unsigned long long *>(handle_scratch(h, sizeof(v)));
+    PF_CUDA(cudaMemsetAsync(out, 0, sizeof(v), h->stream));
+    k_csr_shape<<<grid_for(h, D, 256, 8), 256, 0, h->stream>>>(indptr, indices, D, out);
     PF_CUDA(cudaGetLastError());
     count_launches(1);
-    PF_CUDA(cudaMemcpyAsync(&most, out, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    PF_CUDA(cudaMemcpyAsync(v, out, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
     PF_CUDA(cudaStreamSynchronize(h->stream));
-    return most;
+    CsrShape s;
+    s.max_row = (int)std::min<unsigned long long>(v[0], INT32_MAX);
+    s.slots = 32.0 * (double)v[1];
+    for (int k = 1; k <= 4; ++k) {
+        s.far_entries[k] = (double)v[1 + k];
+        s.far[k] = (double)v[5 + k];
+    }
+    return s;
 }
 
 pf_op *adopt_csr(pf_handle *h, int64_t D, int64_t nnz, int64_t *dptr, int32_t *didx, double *dv64, float *dv32) {
@@ -335,7 +370,7 @@ pf_op *adopt_csr(pf_handle *h, int64_t D, int64_t nnz, int64_t *dptr, int32_t *d
     op->csr64 = {dptr, didx, dv64};
     op->csr32 = {dptr, didx, dv32};
     try {
-        op->max_row = csr_longest_row(h, D, dptr);
+        op->shape = csr_shape(h, D, dptr, didx);
         build_multi_tables(op);
     } catch (...) {
         delete op;
@@ -365,7 +400,7 @@ pf_op *bind_op(const pf_op *src, pf_handle *h) {
     op->csr64 = src->csr64;
     op->csr32 = src->csr32;
     op->nnz = src->nnz;
-    op->max_row = src->max_row;
+    op->shape = src->shape;
     op->complex_dim = src->complex_dim;
     op->d_states = src->d_states;
     op->d_rank_tab = src->d_rank_tab;

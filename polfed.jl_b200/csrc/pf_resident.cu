@@ -886,14 +886,19 @@ static double list_terms(const pf_op *op) {
 }
 
 // The plan of V columns of a chain or CSR operator on 2^clog CTAs, if it fits.
-// us as for qsun_plan (measured: 0.18 ns a row and entry in one CTA, 0.27 ns on
-// several, where a quarter of the entries are remote; CSR values and wider
-// chunks cost a quarter more; 0.4 and 1.2 us for the barrier and latencies).
+// us as for qsun_plan.  Chains (measured): 0.18 ns a row and entry in one CTA,
+// 0.27 ns on several, where a quarter of the entries are remote; wider chunks
+// cost a quarter more; 0.4 and 1.2 us for the barrier and latencies.
+// CSR rows may have their entries anywhere.  Measured over 41 matrices of 200 to
+// 50000 rows (chains, grids, bands, random columns; 3 to 60 entries a row), on
+// several CTAs: 1.3 ns a sector of remote columns, 0.8 ns a row, 0.38 us for each
+// eight entries of a row that wait for remote ones, 1.05 us for the barrier,
+// within a standard deviation of 10 to 15 %; in one CTA the row places alone.
 template <typename T>
 static bool list_plan(const pf_op *op, int V, int clog, bool kpm, ResPlan *p) {
     const bool csr = op->kind == OP_CSR;
     if (!csr && op->chain64.diag == nullptr) return false;
-    const int width = csr ? op->max_row : op->chain64.nb;
+    const int width = csr ? op->shape.max_row : op->chain64.nb;
     const int64_t D = op->dim;
     const int64_t rows = (D + (1 << clog) - 1) >> clog;
     // the last CTA's last row would be kResNone
@@ -916,9 +921,24 @@ static bool list_plan(const pf_op *op, int V, int clog, bool kpm, ResPlan *p) {
     if (p->diag_smem) smem += (size_t)rows * sizeof(T);
     p->smem = smem;
     p->work = (size_t)D * p->groups * (16 + (csr ? 8 * sizeof(T) : 0));
-    const double wide = V * (int)sizeof(T) == 16 ? 1.25 : V * (int)sizeof(T) == 4 ? 0.85 : 1.0;
-    p->busy_us = (double)rows * list_terms(op) * (clog ? 0.27e-3 : 0.18e-3) * wide * (csr ? 1.25 : 1.0);
-    p->us = p->busy_us + (clog ? 1.2 : 0.4);
+    const int bytes = V * (int)sizeof(T);
+    const double wide = bytes == 16 ? 1.25 : bytes == 4 ? 0.85 : 1.0;
+    if (csr) {
+        const CsrShape &sh = op->shape;
+        const double C = 1 << clog, slots = sh.slots / C;
+        if (clog == 0) {
+            p->busy_us = (slots * (bytes == 16 ? 0.18 : bytes == 8 ? 0.115 : 0.08) + (p->list_smem ? 0.0 : 0.4 * rows)) * 1e-3;
+            p->us = p->busy_us + (kpm ? 0.8 : 0.4);
+        } else {
+            p->busy_us = (sh.far[clog] / C * 1.3 + 0.8 * rows +
+                          slots * ((bytes == 16 ? 0.09 : bytes == 8 ? 0.015 : 0.01) + (p->list_smem ? 0.0 : 0.04))) * 1e-3;
+            const double waits = std::ceil((double)rows / p->threads) * p->groups * sh.far_entries[clog] / std::max(1.0, (double)op->nnz);
+            p->us = p->busy_us + (kpm ? 1.3 : 1.05) + 0.38 * waits;
+        }
+    } else {
+        p->busy_us = (double)rows * list_terms(op) * (clog ? 0.27e-3 : 0.18e-3) * wide;
+        p->us = p->busy_us + (clog ? 1.2 : 0.4);
+    }
     if (!csr && !kpm && p->groups <= 3 && rows <= 1024) {
         // measured: 1.35 us for the barrier and the latency of remote rows, 0.042
         // ns a row and entry for every doubling of the CTAs (the remote share
@@ -972,16 +992,43 @@ static int res_resident(const ResPlan &p) {
     return cache[key] = n;
 }
 
-// A filter step of ncol columns by the step kernels, in us: what the autotuned
-// kernels, or a chain's listed ones, measured over D = 2^11 .. 2^17 (a launch
-// floor, then the gathered values).  KPM steps (fused dots) are about twice that.
-static double step_us(const pf_op *op, int ncol, int elem, bool kpm) {
+// A CSR step of s columns, V a thread, in us (measured over the matrices of
+// list_plan): a launch, a dependent gather for every batch of a row, the gathered
+// sectors, the blocks' bytes.
+static double csr_step_us(const pf_op *op, int s, int elem, int V, bool dots) {
+    const int bytes = V * elem, batch = bytes >= 64 ? 2 : bytes >= 16 ? 4 : 8;
+    const double waits = std::ceil((double)op->shape.max_row / batch) * (bytes < 16 ? 0.8 : 0.55);
+    const double sectors = (double)op->nnz * (s / V) * std::max(1.0, bytes / 32.0), moved = (double)op->dim * s * elem;
+    if (dots) return (bytes < 32 ? 3.0 : 4.9) + waits + sectors * (bytes < 32 ? 9e-6 : 2e-6) + moved * 0.7e-6;
+    return (bytes < 64 ? 1.4 : 2.2) + waits + sectors * 3.5e-6 + moved * 0.12e-6;
+}
+
+// A step of ncol columns by the step kernels, in us: what the kernels, autotuned
+// or a chain's listed ones, measured over D = 2^11 .. 2^17 (a launch floor, then
+// the gathered values).  KPM: a step of every block of columns, with fused dots,
+// of chains and the Quantum Sun about twice a filter's.  CSR filters depend on
+// the columns a thread takes: the default, or the best if they are (to be) tuned;
+// a CSR KPM run pays 55 us a block beyond its K steps (its probes and their norms).
+static double step_us(const pf_op *op, int ncol, int elem, bool kpm, int K, bool tuned) {
     const double D = (double)op->dim, w = elem == 8 ? 1.0 : 0.7;
-    double us;
-    if (op->kind == OP_QSUN) us = 2.8 + D * ncol * (op->L_loc + (1 << op->L_grain)) * 0.42e-6 * w;
-    else if (op->kind == OP_CSR) us = 2.8 + D * ncol * list_terms(op) * 1.15e-6 * w;
-    else us = 3.0 + D * ncol * list_terms(op) * 0.9e-6 * (elem == 8 ? 1.0 : 0.5);
-    return kpm ? 2 * us : us;
+    if (op->kind == OP_CSR) {
+        double us = 0.0;
+        if (kpm) {
+            const double block = 55.0 / std::max(K, 1);
+            if (ncol >= 64) us = (ncol / 64) * (block + csr_step_us(op, 64, elem, dots_width(64, elem), true));
+            for (int nb = 32; nb >= 1; nb /= 2)
+                if (ncol % 64 & nb) us += block + csr_step_us(op, nb, elem, dots_width(nb, elem), true);
+            return us;
+        }
+        us = csr_step_us(op, ncol, elem, default_width(ncol, elem), false);
+        if (tuned)
+            for (int V = 1; V * elem <= 64 && ncol % V == 0; V *= 2) us = std::min(us, csr_step_us(op, ncol, elem, V, false));
+        return us;
+    }
+    const int n = kpm ? std::min(ncol, 64) : ncol;
+    const double us = op->kind == OP_QSUN ? 2.8 + D * n * (op->L_loc + (1 << op->L_grain)) * 0.42e-6 * w
+                                          : 3.0 + D * n * list_terms(op) * 0.9e-6 * (elem == 8 ? 1.0 : 0.5);
+    return kpm ? 2 * us * std::ceil(ncol / 64.0) : us;
 }
 
 // A filter of g columns (or groups of columns) with n < g clusters resident runs
@@ -1015,12 +1062,13 @@ static bool kpm_launch(ResPlan *p, int64_t D, int elem, int ncol, int M, int res
 // Of the cluster sizes and widths that fit, the one with the least estimated
 // time for all columns: as many rounds of clusters as are not resident at once,
 // or the SMs' total work where that is more.  K: a filter's order, a KPM run's steps.
+// A CSR matrix has to be ahead by 6 %: of 880 measured filters and KPM runs, the
+// choice then was slower than the step kernels in 4, by 20 % at most (by a model
+// without its columns' places: in 99, by up to a factor of 9).
 template <typename T>
-bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
+bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, bool tuned, ResPlan *best) {
     const double sms = op->h->num_sms;
-    // KPM blocks of the step path hold 64 columns
-    double bt = kpm ? step_us(op, std::min(ncol, 64), sizeof(T), true) * std::ceil(ncol / 64.0)
-                    : step_us(op, ncol, sizeof(T), false);
+    double bt = step_us(op, ncol, (int)sizeof(T), kpm, K, tuned) / (op->kind == OP_CSR ? 1.06 : 1.0);
     bool have = false;
     for (int clog = 0; clog <= 4; ++clog)
         for (int V = 1; V * (int)sizeof(T) <= (op->kind == OP_QSUN ? (int)sizeof(T) : 16); V *= 2) {
@@ -1032,6 +1080,13 @@ bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *best) {
             const int groups = res_groups(p, ncol);
             if (kpm && !kpm_launch(&p, op->dim, (int)sizeof(T), ncol, K, n)) continue;
             double t = std::max((groups + n - 1) / n * p.us, groups * (1 << clog) * p.busy_us / sms);
+            if (op->kind == OP_CSR) {
+                // beyond the clusters that have their SMs to themselves, the next share them
+                ResPlan alone = p;
+                alone.smem = kResSmem;
+                const int n1 = std::max(1, res_resident(alone));
+                t = (groups + n - 1) / n * (p.us - p.busy_us) + (groups + n1 - 1) / n1 * p.busy_us;
+            }
             const bool rotates = op->kind == OP_QSUN || (p.pinned && !op->h->shared);
             if (rotates && !kpm && K > 0 && groups > n) {
                 const int steps = (K + n - 1) / n;
@@ -1190,7 +1245,7 @@ void resident_kpm(pf_op *op, cudaStream_t st, const ResPlan &p, void *work, int 
 }
 
 #define PF_RES_INST(T)                                                                                              \
-    template bool resident_plan<T>(const pf_op *, int, bool, int, ResPlan *);                                         \
+    template bool resident_plan<T>(const pf_op *, int, bool, int, bool, ResPlan *);                                   \
     template void resident_prepare<T>(pf_op *, cudaStream_t, const ResPlan &, void *);                             \
     template void resident_filter<T>(pf_op *, cudaStream_t, const ResPlan &, void *, int, int, const double *,     \
                                      double, double, const T *, int64_t, int64_t, T *, int64_t, int64_t);         \

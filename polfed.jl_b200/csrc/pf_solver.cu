@@ -178,10 +178,16 @@ constexpr int kListSteps = 8;
 // ------------------------------------------------------------ the filter
 // Whether an s-column filter runs whole on chip: it fits and is estimated
 // faster than the step kernels, and the caller asked for neither column slabs
-// nor a step variant of their own.
+// nor a step variant of their own.  tuned: the filter is to have its step kernel
+// autotuned if it runs by steps.
 template <typename T>
-static bool resident_filter_plan(pf_op *op, int s, int K, ResPlan *plan) {
-    return op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T)) && resident_plan<T>(op, s, false, K, plan);
+static bool resident_filter_plan(pf_op *op, int s, int K, bool tuned, ResPlan *plan) {
+    if (op->slab_cols > 0 || pinned_step(op, s, (int)sizeof(T))) return false;
+    if (!tuned) {
+        std::lock_guard<std::mutex> lock(op->tune_mu);
+        tuned = op->tuned_width.count(std::make_pair((int)sizeof(T), s)) > 0;
+    }
+    return resident_plan<T>(op, s, false, K, tuned, plan);
 }
 
 // Y = sum_k c_k T_k(Htilde) X on RI blocks (ClenshawAlgorithm.jl:12-29).
@@ -206,9 +212,9 @@ struct Filter {
     // io = false: only the two work blocks (the filter engine reads and
     // writes the caller's blocks directly)
     Filter(pf_op *op_, int s_, const std::vector<double> &coeffs, double a_, double b_, bool io = true,
-           ListRef lr = {})
+           ListRef lr = {}, bool tuned = false)
         : op(op_), s(s_), K((int)coeffs.size() - 1), c(coeffs), a(a_), b(b_),
-          resident(io && resident_filter_plan<T>(op_, s_, (int)coeffs.size() - 1, &plan)) {
+          resident(io && resident_filter_plan<T>(op_, s_, (int)coeffs.size() - 1, tuned, &plan)) {
         const size_t n = (size_t)op->dim * s;
         if (resident) {
             dc.alloc(c.size());
@@ -330,7 +336,7 @@ static bool kpm_on_chip(pf_op *op, double a, double b, int N, int R, const T *pr
     cudaStream_t st = h->stream;
     const int M = (N - 1 + 1) / 2;
     ResPlan plan;
-    if ((int64_t)(M + 1) * R > ((int64_t)1 << 22) || !resident_plan<T>(op, R, true, M, &plan)) return false;
+    if ((int64_t)(M + 1) * R > ((int64_t)1 << 22) || !resident_plan<T>(op, R, true, M, false, &plan)) return false;
     const size_t sums = (size_t)2 * (M + 1);   // of a probe
     const int some = std::max(1, (int)(kResKpmSums / (sums * sizeof(double)) / plan.launch)) * plan.launch;
     DevArray<unsigned char> work;
@@ -1844,8 +1850,8 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     // is this solve's own CUDA graph of steps, whose kernel is tuned.
     pf_engine *eng = (h->engine && multi_eligible(op, fdtype)) ? h->engine : nullptr;
     ResPlan onchip;
-    const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, (int)coeffs.size() - 1, &onchip)
-                                                 : resident_filter_plan<float>(op, s, (int)coeffs.size() - 1, &onchip));
+    const bool steps = eng || !(fdtype == PF_F64 ? resident_filter_plan<double>(op, s, (int)coeffs.size() - 1, P->autotune != 0, &onchip)
+                                                 : resident_filter_plan<float>(op, s, (int)coeffs.size() - 1, P->autotune != 0, &onchip));
     if (P->autotune && steps && (eng || !list.list || op->slab_cols > 0)) {
         bool have;
         {
@@ -1856,7 +1862,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     }
     const int ew = engine_width(op, s, fdtype == PF_F64 ? 8 : 4);
     if (P->precision == PF_PREC_FP64) {
-        Filter<double> filt(op, s, coeffs, a, b, eng == nullptr, list);
+        Filter<double> filt(op, s, coeffs, a, b, eng == nullptr, list, P->autotune != 0);
         BlockMap fmap = [&](const double *X, double *Y) {
             if (eng) {
                 engine_filter(eng, op, st, 8, s, ew, coeffs, a, b, (void *)X, Y, filt.A.p, filt.B.p);
@@ -1878,7 +1884,7 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
         // last target is the filter ratio P(lambda_{2 nev}) / P(lambda_{nev})
         const int guard = std::max(s, nev);
         {
-            Filter<float> filt(op, s, coeffs, a, b, eng == nullptr, list);
+            Filter<float> filt(op, s, coeffs, a, b, eng == nullptr, list, P->autotune != 0);
             BlockMap fmap = [&](const double *X, double *Y) {
                 launch_ri_to_cm<double, float>(st, (int64_t)D * s, 1, X, filt.x(), (int64_t)D * s);
                 if (eng) engine_filter(eng, op, st, 4, s, ew, coeffs, a, b, filt.x(), filt.y(), filt.A.p, filt.B.p);

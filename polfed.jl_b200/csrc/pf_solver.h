@@ -114,10 +114,10 @@ struct ResPlan {
 // the step kernels' two blocks of 64 columns are less, and of the sums it reads back at once.
 constexpr size_t kResKpmBytes = size_t(512) << 20, kResKpmSums = size_t(16) << 20;
 // The plan for ncol columns of the operator (K: a filter's order, a KPM run's
-// steps); false: none (a column does not fit a cluster, or the step kernels are
-// estimated faster).
+// steps; tuned: the step kernel is, or is about to be, the autotuner's); false:
+// none (a column does not fit a cluster, or the step kernels are estimated faster).
 template <typename T>
-bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, ResPlan *plan);
+bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, bool tuned, ResPlan *plan);
 // Fills the workspace (plan.work bytes) for the operator; once per workspace.
 template <typename T>
 void resident_prepare(pf_op *op, cudaStream_t st, const ResPlan &plan, void *work);

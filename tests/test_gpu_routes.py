@@ -204,3 +204,28 @@ def test_autotune_releases_a_pinned_variant(pkg, cuda):
     pkg.autotune(op, s)
     names = kernels(torch, call)
     assert ran(names, "k_res_pinned") and not ran(names, "k_step"), names
+
+
+# ------------------------------------------------------------ sparse matrices on chip
+
+def _band(pkg, D, k, width, seed):
+    rng = np.random.default_rng(seed)
+    idx = (np.repeat(np.arange(D), k) + rng.integers(-width, width + 1, size=D * k)) % D
+    return pkg.SparseOperator((np.arange(D + 1) * k, idx, rng.standard_normal(D * k)))
+
+
+@pytest.mark.parametrize("D,k,width,s,R", [(12000, 8, 40, 4, 64), (400, 7, 200, 8, 64), (6435, 30, 3217, 8, 64),
+                                           (50000, 15, 25000, 2, 64)])
+def test_sparse_matrices_run_on_chip_where_their_columns_are_near(pkg, cuda, D, k, width, s, R):
+    """Rows whose entries lie in the same CTA, or a matrix that fits a few, run on
+    chip; rows with 30 and 15 entries anywhere do not: a remote read for each
+    made them up to six times slower than the step kernels."""
+    torch = cuda
+    op = _band(pkg, D, k, width, 3)
+    X = _block(torch, D, s, torch.float64, 1)
+    Y = torch.empty_like(X)
+    c = np.cos(np.arange(40))
+    near = 2 * width < D // 16 or D <= 1000
+    for names in (kernels(torch, lambda: pkg.chebyshev_filter(op, Y, X, c, 30.0, 0.1)),
+                  kernels(torch, lambda: pkg.kpm_moments(op, 40, R, 30.0, 0.1, seed=1))):
+        assert ran(names, "k_res_list") == near and ran(names, "k_step") != near, names
