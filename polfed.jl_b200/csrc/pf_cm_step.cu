@@ -167,23 +167,55 @@ static void launch_cm(pf_op *op, cudaStream_t st, const ChainDesc<T> &ch, const 
     else launch_cm<T>(op, st, cs, a, 0);
 }
 
+// Whether this form is at most as slow as copies and row gathers, whose gathers
+// of wide blocks of many rows fill whole sectors only in the row-interleaved
+// layout.  The lines lie where the two times, measured on a B200 over the widths
+// 2 .. 64 and both types, cross.
+//
+// Chains: J1-J2 L = 22, s = 8 FP64 254 us staged, 355 here; XXZ L = 20, s = 3
+// recurrence 115 and 57.
+//
+// Quantum Sun (2^6 .. 2^23 states), by the grain, whose dense block costs its
+// rows' reads once a column: up to `narrow` columns at any size; up to `wide`
+// columns, or any number, in blocks of so many elements.  Recurrences 2^16, s = 8
+// FP64 55 us staged and 38 here; applies of a 4-site grain with 2^22 states, s =
+// 16 FP32 996 staged, 2243 here.  An odd number of columns is staged one column
+// a thread: here it is faster except for FP64 applies of a 4-site grain.
+//
+// CSR (200 to 1.5 million rows; chains, grids, bands, random columns): by the
+// sectors gathered beyond the staged form's, those near the row at 0.3 (they
+// mostly hit L1), against the copies: a number that pays for their launches, or
+// one a row.  24310 rows of a chain, s = 8 recurrence 44 and 32 us; 50000 rows of
+// 15 entries anywhere, s = 12 apply 46 and 72.
+static bool cm_worth(const pf_op *op, int s, int elem, bool rec) {
+    const double n = (double)op->dim * s;
+    const int width = s * elem, fp32 = elem == 4;
+    if (op->kind == OP_CHAIN) return width <= (rec ? 32 : 24) || n <= 400000;
+    if (op->kind == OP_QSUN) {
+        struct Lines { int narrow, wide; double wide_n, any_n; };
+        static const Lines lines[2][2][3] = {   // apply, recurrence; FP64, FP32; grains of up to 2, of 3 and 4 sites
+            {{{8, 8, 0, 1.6e6}, {4, 8, 4.3e6, 0.8e6}, {0, 4, 2.1e6, 0.27e6}},
+             {{12, 16, 2.2e6, 1.1e6}, {6, 8, 17e6, 1.06e6}, {4, 4, 0, 0.3e6}}},
+            {{{8, 8, 0, 1.6e6}, {8, 8, 0, 1.6e6}, {4, 8, 2.2e6, 0.8e6}},
+             {{16, 16, 0, 1.6e6}, {12, 16, 8.4e6, 1.6e6}, {6, 8, 8.4e6, 0.8e6}}}};
+        const int g = std::max(op->L_grain, 2) - 2;
+        const Lines &l = lines[rec][fp32][g];
+        if (s % 2 == 1 && (g < 2 || rec || fp32)) return width <= 64 || n <= 1.6e6;
+        return s <= l.narrow || (s <= l.wide && n <= l.wide_n) || n <= l.any_n;
+    }
+    if (width > 32 && n > 600000) return false;
+    static const double few[2][2] = {{1.2e6, 1.8e6}, {2.4e6, 3.0e6}}, per_row[2][2] = {{25, 30}, {42, 60}};
+    const double load = op->shape.far[4] + 0.3 * (op->shape.sectors - op->shape.far[4]);
+    return load * (s - 1) <= std::max(few[rec][fp32], per_row[rec][fp32] * (double)op->dim);
+}
+
 template <typename T>
 bool launch_step_cm(pf_op *op, cudaStream_t st, int s, const T *q, const T *p, const T *x, T *out, int64_t ld,
                     int64_t ldout, double cx, double alpha, double beta, double inva, double shift) {
     const int64_t D = op->dim;
     if (s < 2 || (op->kind == OP_CHAIN && op->chain64.diag == nullptr)) return false;
     if ((s - 1) / cm_columns(D, s) >= 65535) return false;   // more blocks of columns than a grid's second dimension has
-    // Where copies and row gathers are faster: wide blocks of many rows, whose
-    // gathers fill whole sectors only in the row-interleaved layout (J1-J2 L = 22,
-    // s = 8 FP64: 254 us staged, 355 here; Quantum Sun 2^18, s = 24: 148 and 170).
-    // Below these lines this form was never slower (recurrence: Quantum Sun 2^16
-    // s = 8 FP64 55 -> 38, 2^18 123 -> 77, XXZ L = 20 s = 3 115 -> 57, CSR 24310
-    // rows s = 8 44 -> 32).
-    const int64_t n = D * s, width = (int64_t)s * sizeof(T);
-    const bool worth = op->kind == OP_QSUN  ? width <= 64 || n <= 1600000
-                       : op->kind == OP_CSR ? width <= 32 || n <= 600000
-                                            : width <= (p ? 32 : 24) || n <= 400000;
-    if (!worth) return false;
+    if (!cm_worth(op, s, (int)sizeof(T), p != nullptr)) return false;
     // the output may be p or x itself (each element is read, then written, by
     // one thread), but not overlap q, or p or x at another place
     const size_t in = ((size_t)(s - 1) * ld + D) * sizeof(T), o = ((size_t)(s - 1) * ldout + D) * sizeof(T);

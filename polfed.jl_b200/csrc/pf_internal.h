@@ -104,10 +104,10 @@ struct CsrDesc {
 // rows; its n-th gather is the n-th entry of each of its rows.
 struct CsrShape {
     int max_row = 0;           // entries of the longest row
+    double sectors = 0;        // sectors of 32 bytes (four FP64 columns) a gather reads, counted per gather
     double slots = 0;          // row places of all slices, their rows as long as the longest, in eights
     // of a split of the rows into 2^k equal ranges: entries whose column is not
-    // in their row's range, and the sectors of 32 bytes (four FP64 columns) these
-    // are gathered from, counted per gather
+    // in their row's range, and the sectors of these
     double far_entries[5] = {}, far[5] = {};
 };
 

@@ -297,12 +297,12 @@ pf_op *create_csr_hermitian(pf_handle *h, int64_t D, int64_t nnz, const int64_t 
 }
 
 // CsrShape, counted on the device: a warp per slice.  out: max_row, slots / 32,
-// far_entries[1..4], far[1..4].
+// far_entries[1..4], far[1..4], sectors.
 static __global__ void k_csr_shape(const int64_t *__restrict__ indptr, const int32_t *__restrict__ indices, int64_t D,
                                    unsigned long long *out) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
-    unsigned long long most = 0, slots = 0, fe[5] = {0, 0, 0, 0, 0}, fs[5] = {0, 0, 0, 0, 0};
+    unsigned long long most = 0, slots = 0, sectors = 0, fe[5] = {0, 0, 0, 0, 0}, fs[5] = {0, 0, 0, 0, 0};
     for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 32; w * 32 < D; w += warps) {
         const int64_t row = w * 32 + lane;
         const int64_t p = row < D ? indptr[row] : 0;
@@ -313,6 +313,7 @@ static __global__ void k_csr_shape(const int64_t *__restrict__ indptr, const int
         for (unsigned n = 0; n < longest; ++n) {
             const uint32_t col = n < cnt ? (uint32_t)indices[p + n] : 0xffffffffu;
             const unsigned same = __match_any_sync(0xffffffffu, col >> 2);
+            sectors += __popc(__ballot_sync(0xffffffffu, n < cnt && same >> lane == 1u));
 #pragma unroll
             for (int k = 1; k <= 4; ++k) {
                 const uint32_t range = (uint32_t)((D + (1 << k) - 1) >> k);
@@ -329,11 +330,12 @@ static __global__ void k_csr_shape(const int64_t *__restrict__ indptr, const int
             atomicAdd(out + 1 + k, fe[k]);
             atomicAdd(out + 5 + k, fs[k]);
         }
+        atomicAdd(out + 10, sectors);
     }
 }
 
 static CsrShape csr_shape(pf_handle *h, int64_t D, const int64_t *indptr, const int32_t *indices) {
-    unsigned long long v[10] = {};
+    unsigned long long v[11] = {};
     auto *out = static_cast<unsigned long long *>(handle_scratch(h, sizeof(v)));
     PF_CUDA(cudaMemsetAsync(out, 0, sizeof(v), h->stream));
     k_csr_shape<<<grid_for(h, D, 256, 8), 256, 0, h->stream>>>(indptr, indices, D, out);
@@ -344,6 +346,7 @@ static CsrShape csr_shape(pf_handle *h, int64_t D, const int64_t *indptr, const 
     CsrShape s;
     s.max_row = (int)std::min<unsigned long long>(v[0], INT32_MAX);
     s.slots = 32.0 * (double)v[1];
+    s.sectors = (double)v[10];
     for (int k = 1; k <= 4; ++k) {
         s.far_entries[k] = (double)v[1 + k];
         s.far[k] = (double)v[5 + k];

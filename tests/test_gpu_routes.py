@@ -229,3 +229,25 @@ def test_sparse_matrices_run_on_chip_where_their_columns_are_near(pkg, cuda, D, 
     for names in (kernels(torch, lambda: pkg.chebyshev_filter(op, Y, X, c, 30.0, 0.1)),
                   kernels(torch, lambda: pkg.kpm_moments(op, 40, R, 30.0, 0.1, seed=1))):
         assert ran(names, "k_res_list") == near and ran(names, "k_step") != near, names
+
+
+# ------------------------------------------------------------ one step on column-major blocks
+
+def test_steps_are_staged_where_that_is_faster(pkg, cuda):
+    """Column-major steps on either side of the rule's lines: a wide apply of a
+    4-site grain (2.3 times slower column-major), a matrix with 15 entries a row
+    anywhere, the same sizes with a narrow block, a smaller grain or near columns."""
+    torch = cuda
+    rng = np.random.default_rng(5)
+    far = pkg.SparseOperator((np.arange(50001) * 15, rng.integers(0, 50000, size=50000 * 15), rng.standard_normal(50000 * 15)))
+    idx = (np.repeat(np.arange(50000), 8) + rng.integers(-300, 301, size=400000)) % 50000
+    near = pkg.SparseOperator((np.arange(50001) * 8, np.sort(idx.reshape(-1, 8), axis=1).ravel(), rng.standard_normal(400000)))
+    cases = [(_qsun(pkg, 14, 4, 1), 16, torch.float32, False), (_qsun(pkg, 14, 4, 1), 4, torch.float32, True),
+             (_qsun(pkg, 15, 3, 1), 8, torch.float64, True), (far, 12, torch.float64, False), (far, 2, torch.float64, True),
+             (near, 8, torch.float64, True), (_chain(pkg, 16, 8, 1), 8, torch.float64, True),
+             (_chain(pkg, 20, 10, 1), 8, torch.float64, False)]
+    for op, s, dtype, direct in cases:
+        X = _block(torch, op.dim, s, dtype, 1)
+        Y = torch.empty_like(X)
+        names = kernels(torch, lambda: pkg.apply(op, Y, X, 3.0, 0.1))
+        assert ran(names, "k_step_cm") == direct and ran(names, "k_step") != direct, (op.dim, s, names)
