@@ -892,8 +892,9 @@ static double list_terms(const pf_op *op) {
 // CSR rows may have their entries anywhere.  Measured over 41 matrices of 200 to
 // 50000 rows (chains, grids, bands, random columns; 3 to 60 entries a row), on
 // several CTAs: 1.3 ns a sector of remote columns, 0.8 ns a row, 0.38 us for each
-// eight entries of a row that wait for remote ones, 1.05 us for the barrier,
-// within a standard deviation of 10 to 15 %; in one CTA the row places alone.
+// eight entries of a row that wait for remote ones, as much for each eight read
+// from a list in L2, 1.05 us for the barrier, within a standard deviation of 10 to
+// 15 %; in one CTA the row places alone.
 template <typename T>
 static bool list_plan(const pf_op *op, int V, int clog, bool kpm, ResPlan *p) {
     const bool csr = op->kind == OP_CSR;
@@ -930,10 +931,10 @@ static bool list_plan(const pf_op *op, int V, int clog, bool kpm, ResPlan *p) {
             p->busy_us = (slots * (bytes == 16 ? 0.18 : bytes == 8 ? 0.115 : 0.08) + (p->list_smem ? 0.0 : 0.4 * rows)) * 1e-3;
             p->us = p->busy_us + (kpm ? 0.8 : 0.4);
         } else {
-            p->busy_us = (sh.far[clog] / C * 1.3 + 0.8 * rows +
-                          slots * ((bytes == 16 ? 0.09 : bytes == 8 ? 0.015 : 0.01) + (p->list_smem ? 0.0 : 0.04))) * 1e-3;
-            const double waits = std::ceil((double)rows / p->threads) * p->groups * sh.far_entries[clog] / std::max(1.0, (double)op->nnz);
-            p->us = p->busy_us + (kpm ? 1.3 : 1.05) + 0.38 * waits;
+            p->busy_us = (sh.far[clog] / C * 1.3 + 0.8 * rows + slots * (bytes == 16 ? 0.09 : bytes == 8 ? 0.015 : 0.01)) * 1e-3;
+            const double turns = std::ceil((double)rows / p->threads), entries = std::max(1.0, (double)op->nnz);
+            p->us = p->busy_us + (kpm ? 1.3 : 1.05) + 0.38 * turns * p->groups * sh.far_entries[clog] / entries;
+            if (!p->list_smem) p->us += turns * sh.slots / 8 / (double)D * (sizeof(T) == 4 ? 0.25 : V == 1 ? 0.45 : 0.75);
         }
     } else {
         p->busy_us = (double)rows * list_terms(op) * (clog ? 0.27e-3 : 0.18e-3) * wide;
@@ -1007,7 +1008,8 @@ static double csr_step_us(const pf_op *op, int s, int elem, int V, bool dots) {
 // or a chain's listed ones, measured over D = 2^11 .. 2^17 (a launch floor, then
 // the gathered values).  KPM: a step of every block of columns, with fused dots,
 // of chains and the Quantum Sun about twice a filter's.  CSR filters depend on
-// the columns a thread takes: the default, or the best if they are (to be) tuned;
+// the columns a thread takes: the default, or the best if they are (to be) tuned
+// (whose gather batch saves a fifth more);
 // a CSR KPM run pays 55 us a block beyond its K steps (its probes and their norms).
 static double step_us(const pf_op *op, int ncol, int elem, bool kpm, int K, bool tuned) {
     const double D = (double)op->dim, w = elem == 8 ? 1.0 : 0.7;
@@ -1022,7 +1024,7 @@ static double step_us(const pf_op *op, int ncol, int elem, bool kpm, int K, bool
         }
         us = csr_step_us(op, ncol, elem, default_width(ncol, elem), false);
         if (tuned)
-            for (int V = 1; V * elem <= 64 && ncol % V == 0; V *= 2) us = std::min(us, csr_step_us(op, ncol, elem, V, false));
+            for (int V = 1; V * elem <= 64 && ncol % V == 0; V *= 2) us = std::min(us, 0.8 * csr_step_us(op, ncol, elem, V, false));
         return us;
     }
     const int n = kpm ? std::min(ncol, 64) : ncol;
