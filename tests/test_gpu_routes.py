@@ -251,3 +251,151 @@ def test_steps_are_staged_where_that_is_faster(pkg, cuda):
         Y = torch.empty_like(X)
         names = kernels(torch, lambda: pkg.apply(op, Y, X, 3.0, 0.1))
         assert ran(names, "k_step_cm") == direct and ran(names, "k_step") != direct, (op.dim, s, names)
+
+
+# ------------------------------------------------------------ every on-chip filter form, by name
+
+def _xxz_csr(pkg, L, k):
+    """The matrix of an XXZ chain's sector, rows cut to at most k entries (in storage order)."""
+    st = np.array([s for s in range(1 << L) if bin(s).count("1") == L // 2])
+    rows, cols = [np.arange(len(st))], [np.arange(len(st))]
+    for a in range(L):
+        m = (1 << a) | (1 << (a + 1) % L)
+        on = np.nonzero((st & m) * (st & m ^ m))[0]
+        rows.append(on)
+        cols.append(np.searchsorted(st, st[on] ^ m))
+    r, c = np.concatenate(rows), np.concatenate(cols)
+    o = np.lexsort((c, r))
+    r, c = r[o], c[o]
+    keep = np.arange(len(r)) - np.searchsorted(r, r) < k
+    r, c = r[keep], c[keep]
+    return pkg.SparseOperator((np.searchsorted(r, np.arange(len(st) + 1)), c, np.random.default_rng(L).standard_normal(len(c))))
+
+
+# (operator, columns, dtype, the kernel's name with its first template arguments): the forms' widths, a column count
+# that the width does not divide, one CTA and several, rows of more entries or more rows a CTA than a thread's registers take
+FORMS = {
+    "pinned_1": (lambda p: _chain(p, 14, 7, 1), 1, "fp64", "k_res_pinned<double, 1,"),
+    "pinned_2": (lambda p: _chain(p, 15, 7, 1), 41, "fp64", "k_res_pinned<double, 2,"),
+    "pinned_rotating": (lambda p: _chain(p, 16, 8, 1), 7, "fp64", "k_res_pinned<double, 1,"),
+    "pinned_fp32_2": (lambda p: _chain(p, 14, 7, 1), 41, "fp32", "k_res_pinned<float, 2,"),
+    "pinned_fp32_4": (lambda p: _chain(p, 15, 7, 1), 41, "fp32", "k_res_pinned<float, 4,"),
+    "list_28_bonds": (lambda p: _chain(p, 14, 7, 2, 2), 1, "fp64", "k_res_list<double, 1, false, false>"),
+    "list_28_bonds_wide": (lambda p: _chain(p, 14, 7, 2, 2), 21, "fp64", "k_res_list<double, "),
+    "list_28_bonds_fp32": (lambda p: _chain(p, 14, 7, 2, 2), 43, "fp32", "k_res_list<float, "),
+    "csr_1": (lambda p: _xxz_csr(p, 14, 64), 3, "fp64", "k_res_list<double, 1, true, false>"),
+    "csr_2": (lambda p: _xxz_csr(p, 13, 9), 41, "fp64", "k_res_list<double, 2, true, false>"),
+    "csr_fp32_4": (lambda p: _xxz_csr(p, 14, 64), 43, "fp32", "k_res_list<float, 4, true, false>"),
+    "csr_one_cta": (lambda p: _xxz_csr(p, 10, 64), 7, "fp64", "k_res_list<double, 1, true, false>"),
+    "qsun_one_cta": (lambda p: _qsun(p, 8, 3, 1), 5, "fp64", "k_res_qsun<double, 3, false>"),
+    "qsun_rotating": (lambda p: _qsun(p, 13, 3, 1), 9, "fp64", "k_res_qsun<double, 3, false>"),
+    "qsun_grain_4": (lambda p: _qsun(p, 12, 4, 1), 8, "fp64", "k_res_qsun<double, 4, false>"),
+    "qsun_fp32": (lambda p: _qsun(p, 13, 2, 1), 9, "fp32", "k_res_qsun<float, 2, false>"),
+}
+
+
+@pytest.mark.parametrize("name", list(FORMS))
+def test_filter_on_chip_equals_the_steps(pkg, cuda, name):
+    """The form runs, and gives the pinned step kernels' bits."""
+    torch = cuda
+    make, s, dtype, kernel = FORMS[name]
+    op, ref = make(pkg), make(pkg)
+    pkg.set_step_width(ref, s, 1, dtype)
+    X = _block(torch, op.dim, s, torch.float64 if dtype == "fp64" else torch.float32, 4)
+    Y, Z = torch.full_like(X, math.nan), torch.empty_like(X)
+    for K in (41, 3):
+        c = np.cos(np.arange(K + 1) * 0.6) / (K + 1)
+        names = kernels(torch, lambda: pkg.chebyshev_filter(op, Y, X, c, 21.0, -0.3))
+        assert any(kernel in n for n in names), names
+        assert ran(kernels(torch, lambda: pkg.chebyshev_filter(ref, Z, X, c, 21.0, -0.3)), "k_step")
+        assert torch.equal(Y, Z), (K, float((Y - Z).abs().max()))
+
+
+# ------------------------------------------------------------ moments by steps
+
+@pytest.mark.parametrize("dtype", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind", ["qsun_small", "qsun_large", "csr"])
+def test_moments_by_steps(pkg, cuda, kind, dtype):
+    """The fused-dots step of operators no cluster holds (or too small for one):
+    against the recurrence built from single steps (2 D eps of |v|^2, D <= 2^18:
+    1.2e-10), and the same bits with and without the steps' launch overlap."""
+    torch = cuda
+    rng = np.random.default_rng(2)
+    op = {"qsun_small": lambda: _qsun(pkg, 4, 1, 1), "qsun_large": lambda: _qsun(pkg, 16, 2, 1),
+          "csr": lambda: pkg.SparseOperator((np.arange(901) * 70, rng.integers(0, 900, size=63000), rng.standard_normal(63000) / 8))}[kind]()
+    D, R, N, a, b = op.dim, 11, 14, 30.0, 0.1
+    P = _block(torch, D, R, torch.float64 if dtype == "fp64" else torch.float32, 3) / math.sqrt(D)
+    P = P.t().contiguous().t()
+    call = lambda: pkg.kpm_moments(op, N, R, a, b, probes=P)
+    if not (kind == "qsun_large" and dtype == "fp32"):
+        names = kernels(torch, call)
+        assert ran(names, "k_step") and not ran(names, "k_res_qsun") and not ran(names, "k_res_list"), names
+    got = call()
+    try:
+        pkg.set_launch_overlap(False)
+        assert np.array_equal(got, call())
+    finally:
+        pkg.set_launch_overlap(True)
+    dot = lambda x, y: float((x.double() * y.double()).sum())
+    prev, cur = P, pkg.apply(op, torch.empty_like(P), P, a, b)
+    m0, m1 = dot(prev, prev), dot(cur, prev)
+    want, zero = [m0, m1], torch.zeros_like(P)
+    for _ in range(N // 2):
+        want.append(2 * dot(cur, cur) - m0)
+        nxt = pkg.clenshaw_recurrence(op, torch.empty_like(P), cur, prev, 0.0, zero, a, b)
+        want.append(2 * dot(nxt, cur) - m1)
+        prev, cur = cur, nxt
+    assert np.max(np.abs(got - np.array(want[:N]) * D / R)) <= 4 * 1.2e-10 * m0 * D / R
+
+
+# ------------------------------------------------------------ the start block
+
+def _start(kind, D, s, rng):
+    x = rng.standard_normal((D, s))
+    if kind == "near":            # the last column 1e-5 from the first: inside what CholQR2 takes
+        x[:, -1] = x[:, 0] + 1e-5 * x[:, -1]
+    elif kind == "dependent":     # beyond it: the Householder form decides
+        x[:, -1] = x[:, 0] + 1e-9 * x[:, -1]
+    elif kind == "scaled":
+        x *= 10.0 ** rng.integers(-6, 7, size=s)
+    elif kind == "tiny":
+        x *= 1e-20
+    elif kind == "orthonormal":
+        x = np.linalg.qr(x)[0]
+    return x
+
+
+@pytest.mark.parametrize("s", [1, 5])
+@pytest.mark.parametrize("kind", ["plain", "near", "dependent", "scaled", "tiny", "orthonormal"])
+def test_start_block_spans_what_it_is_given(pkg, cuda, kind, s):
+    """Eigenvalues from a start block, host or device, are those from numpy's
+    orthonormal factor of it: the block's span is kept, whichever form
+    orthonormalises it."""
+    torch = cuda
+    op = _chain(pkg, 10, 5, 3)
+    x = _start(kind, op.dim, s, np.random.default_rng(6))
+    q = np.linalg.qr(x)[0]
+    kw = dict(fact=pkg.FactorizationConfig(tol=1e-13, eigentol=1e-10), dos=pkg.DoSConfig(seed=1), vecs=False)
+    want = np.asarray(pkg.polfed(op, q if s > 1 else q[:, 0], 6, ("rescaled", 0.4), **kw)[0])
+    for start in (x, torch.from_numpy(np.ascontiguousarray(x.T)).cuda().t()):
+        got = np.asarray(pkg.polfed(op, start if s > 1 else start[:, 0], 6, ("rescaled", 0.4), **kw)[0])
+        assert len(got) == len(want) >= 6 and np.max(np.abs(got - want)) < 1e-9
+
+
+def test_start_block_refusals(pkg, cuda):
+    """Entries that are not finite and a zero vector are refused, a zero column is replaced."""
+    from polfed_b200 import _lib
+    op = _chain(pkg, 10, 5, 3)
+    rng = np.random.default_rng(7)
+    kw = dict(dos=pkg.DoSConfig(seed=1), vecs=False)
+    for s in (1, 4):
+        for bad in (math.nan, math.inf):
+            x = rng.standard_normal((op.dim, s))
+            x[17, -1] = bad
+            with pytest.raises((_lib.PolfedArgumentError, ValueError)):
+                pkg.polfed(op, x if s > 1 else x[:, 0], 4, ("rescaled", 0.4), **kw)
+    with pytest.raises((_lib.PolfedArgumentError, ValueError)):
+        pkg.polfed(op, np.zeros(op.dim), 4, ("rescaled", 0.4), **kw)
+    x = rng.standard_normal((op.dim, 3))
+    x[:, 1] = 0.0
+    pkg.polfed(op, x, 4, ("rescaled", 0.4), **kw)
