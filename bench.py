@@ -281,11 +281,8 @@ def run_ours(args, rank, world, local_rank):
     ops, x0s = make_realisations(pkg, nsteps * B, rank_seed0(rank), device=local_rank)
     handle = _lib.handle(local_rank)
     stream = torch.cuda.ExternalStream(_lib.stream_of(handle), device=dev)
-    # set-up outside the timed region: device descriptors, tuned step width, device x0,
-    # worker handles (one stream each) for the batched solves
-    width, _ = pkg.autotune(ops[0], WORKLOAD["blocksize"], "fp64")
-    for o in ops[1:]:
-        pkg.autotune(o, WORKLOAD["blocksize"], "fp64")
+    # set-up outside the timed region: device descriptors, device x0, worker handles
+    # (one stream each) for the batched solves
     x0_dev = []
     for x in x0s:
         t = pkg.col_major(x.shape[0], x.shape[1], device=local_rank)
@@ -407,15 +404,18 @@ def run_ours(args, rank, world, local_rank):
         "config": dict(WORKLOAD, **{"l2": "256 MB buffer written between steps (inside the timed region)",
                                     "step": f"a batch of {B} full POLFED solves in flight together, "
                                             f"one per worker stream",
-                                    "batch": B, "parallelism": f"replicas x{world}", "step_width": width,
-                                    "step_profile": pkg.step_profile(ops[0], WORKLOAD["blocksize"])}),
+                                    "batch": B, "parallelism": f"replicas x{world}",
+                                    "filter_form": "on chip (k_res_qsun); the autotuned step variants are not used"}),
         "e2e": {"value": e_value, "unit": "eigenpairs/s", "h2d_bytes_per_step": B * D * s * 8,
                 "d2h_bytes_per_step": int(statistics.mean(e_nconv) * B * (D * 8 + 8)), "wall_seconds": e_wall},
         "single_solve": {"value": single_value, "unit": "eigenpairs/s",
                          "note": "one solve at a time on one stream (the plain single-solve form)"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "k_res_qsun (Clenshaw recurrence on chip, per step)", "achieved": achieved,
+        "roofline": {"bound": "shared memory, the L2 exchange and the cluster barrier (DRAM at 0.8-2.2 % in the profile)",
+                     "kernel": "k_res_qsun (Clenshaw recurrence on chip, per step)", "achieved": achieved,
                      "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
+                     "note": "achieved is HBM-equivalent: the bytes a step kernel would stream over the step's time; "
+                             "on chip they are not moved, so frac is no share of a bound",
                      "traffic": read_traffic(), "algorithmic_bytes_per_launch": alg_bytes,
                      "avg_launch_us": avg_step * 1e6,
                      "measured_in": "the single-solve runs (library CUDA-event stage timers)",
@@ -425,7 +425,7 @@ def run_ours(args, rank, world, local_rank):
                                            "reads (64 B each) may exceed the measured random-row gather "
                                            "throughput of an L2-resident block (pf_gather_peak)"},
                      "kpm": {"kernel": "k_res_qsun (KPM doubling steps on chip, dots fused)",
-                             "algorithmic_bytes_per_solve": kpm_bytes,
+                             "algorithmic_bytes_per_solve": kpm_bytes, "note": "HBM-equivalent, as above",
                              "achieved": kpm_bytes / kpm_sec / 1e9, "frac": kpm_bytes / kpm_sec / 1e9 / peak,
                              "seconds_per_solve": kpm_sec,
                              "measured_in": "the single-solve runs (library stage timer 'dos')"}},
@@ -713,7 +713,6 @@ def run_c3(args, local_rank):
     op = pkg.j1j2_hamiltonian(24, 12, 1.0, 0.5, 1.0, 1.0, 1.0, rng=rng, device=local_rank)
     D, s, nev = op.dim, C3["blocksize"], C3["nev"]
     x0 = np.asfortranarray(rng.random((D, s)))
-    pkg.autotune(op, s, "fp64")
     sampler = ClockSampler(local_rank)
     sampler.start()
     t0 = time.perf_counter()
@@ -747,19 +746,15 @@ def run_c3(args, local_rank):
 
 def profile_step(width=None, profile=0):
     """Two order-30 Chebyshev filters on one realisation of the workload's
-    operator (s = 8, FP64) with the autotuned step, or with the given step
-    width and profile (the autotuner's timings are not those of a run under
-    ncu, which serialises every launch): a small, bounded case for ncu
-    captures of the step kernel."""
+    operator (s = 8, FP64) on chip, or by steps of the given width and profile:
+    a small, bounded case for ncu captures of either kernel."""
     import numpy as np
     import torch
     import __graft_entry__ as ge
     pkg = ge.load_package()
     ops, x0s = make_realisations(pkg, 1, 1000)
     op = ops[0]
-    if width is None:
-        width, _ = pkg.autotune(op, WORKLOAD["blocksize"], "fp64")
-    else:
+    if width is not None:
         pkg.set_step_width(op, WORKLOAD["blocksize"], width, "fp64", profile)
     D, s = op.dim, WORKLOAD["blocksize"]
     X = pkg.col_major(D, s)
@@ -768,14 +763,14 @@ def profile_step(width=None, profile=0):
     c = np.cos(np.arange(31) * 1.0) * 0.05
     torch.cuda.synchronize()
     # the filters run inside an NVTX range "filters", so a capture can leave
-    # out the autotuner's timing launches (ncu --nvtx --nvtx-include filters/)
+    # out the set-up's launches (ncu --nvtx --nvtx-include filters/)
     torch.cuda.nvtx.range_push("filters")
     for _ in range(2):
         pkg.chebyshev_filter(op, Y, X, c, a=8.0, b=0.0)
     torch.cuda.synchronize()
     torch.cuda.nvtx.range_pop()
-    print(json.dumps({"profile_step": True, "D": D, "s": s, "width": width,
-                      "profile": pkg.step_profile(op, s), "norm": float(Y.norm())}))
+    print(json.dumps({"profile_step": True, "D": D, "s": s, "width": width, "norm": float(Y.norm()),
+                      "profile": None if width is None else pkg.step_profile(op, s)}))
     return 0
 
 
@@ -904,6 +899,8 @@ def step_sweep(large_only=False):
         D = op.dim
         for dt, tdt, w in (("fp64", torch.float64, 8), ("fp32", torch.float32, 4)):
             width, tune = pkg.autotune(op, s, dt)
+            # the step kernel is what is timed: pinned, so that the filter runs by steps
+            pkg.set_step_width(op, s, width, dt, pkg.step_profile(op, s, dt))
             X = pkg.col_major(D, s, dtype=tdt)
             X.copy_(torch.rand(D, s, dtype=tdt, device="cuda:0"))
             Y = pkg.col_major(D, s, dtype=tdt)
@@ -988,8 +985,8 @@ def main():
     ap.add_argument("--profile-step", action="store_true",
                     help="only run two short Chebyshev filters on one realisation (a bounded case for ncu)")
     ap.add_argument("--step-width", type=int, default=None,
-                    help="with --profile-step / --profile-step-large: this step width (columns per thread) "
-                         "instead of the autotuner's")
+                    help="with --profile-step / --profile-step-large: by steps of this width (columns per "
+                         "thread) instead of on chip / the autotuner's")
     ap.add_argument("--step-profile", type=int, default=0, help="with --step-width: the step profile")
     ap.add_argument("--apply-sweep", action="store_true",
                     help="single-vector XXZ H-apply at L=18..24 (the reference's published timings)")
