@@ -129,32 +129,20 @@ static void sync(pf_handle *h) { PF_CUDA(cudaStreamSynchronize(h->stream)); }
 // it lives; empty for other operators and where it would take more than a
 // sixteenth of the device's memory (or does not fit): the steps then rank their
 // flips themselves.
-static void device_bytes(int device, double *total, double *available) {
+static double device_bytes(int device) {
+    thread_local std::map<int, double> known;
+    auto it = known.find(device);
+    if (it != known.end()) return it->second;
     size_t free_b = 0, total_b = 0;
-    cudaMemPool_t pool;
-    uint64_t held = 0, used = 0;
     PF_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    PF_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
-    PF_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
-    PF_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
-    *total = (double)total_b;
-    *available = (double)free_b + (double)(held - std::min(held, used));
+    return known[device] = (double)total_b;
 }
-// Lists of at most this many bytes are made without asking for the device's
-// memory (two driver calls): a solve's footprint has more slack than that.
-constexpr size_t kSmallList = size_t(32) << 20;
 struct ChainList {
     DevArray<unsigned char> mem;
     const void *get() const { return mem.p; }
-    // rest: bytes that the call allocates after the list, which must still fit
-    void make(pf_op *op, cudaStream_t st, double rest) {
+    void make(pf_op *op, cudaStream_t st) {
         const size_t bytes = chain_list_bytes(op);
-        if (bytes == 0 || mem.p) return;
-        if (bytes > kSmallList) {
-            double total, available;
-            device_bytes(op->h->device, &total, &available);
-            if ((double)bytes > total / 16 || (double)bytes + rest > available) return;
-        }
+        if (bytes == 0 || mem.p || (double)bytes > device_bytes(op->h->device) / 16) return;
         try {
             mem.alloc(bytes);
         } catch (const Error &e) {
@@ -166,11 +154,29 @@ struct ChainList {
     }
 };
 // The list of the call that a step, filter or probe belongs to: null with own =
-// false where that call decided to hold none.
+// false where that call holds none.
 struct ListRef {
     const void *list = nullptr;
     bool own = true;   // no such call: it may make its own
 };
+// call(list use) of a call whose list is made before its other memory: if that
+// does not fit the device, once more without a list.  (Asking for the free memory
+// first would cost every call 1 to 4 ms.)
+template <typename Call>
+static void without_list_on_nomem(const pf_op *op, Call call) {
+    if (chain_list_bytes(op) == 0) {
+        call(ListRef{});
+        return;
+    }
+    try {
+        call(ListRef{});
+        return;
+    } catch (const Error &e) {
+        if (e.code != PF_ERR_NOMEM) throw;
+        cudaGetLastError();
+    }
+    call(ListRef{nullptr, false});
+}
 // Steps from which a call makes its own list: making it takes about as long as
 // one step with it, and a step with it two thirds of one without.
 constexpr int kListSteps = 8;
@@ -232,7 +238,7 @@ struct Filter {
         if (io && op->slab_cols <= 0 && !pinned_step(op, s, (int)sizeof(T))) {
             list = lr.list;
             if (lr.own && K >= kListSteps) {
-                own_list.make(op, op->h->stream, 0.0);
+                own_list.make(op, op->h->stream);
                 list = own_list.get();
             }
         }
@@ -405,7 +411,7 @@ static std::vector<double> kpm_moments(pf_op *op, double a, double b, int N, int
     ChainList own_list;
     const void *list = lr.list;
     if (lr.own && (int64_t)M * ((R + 63) / 64) >= kListSteps) {
-        own_list.make(op, st, 0.0);
+        own_list.make(op, st);
         list = own_list.get();
     }
     auto step = [&](int nb, const T *q, const T *p, T *out, double alpha, double beta, int flags, double *dst) {
@@ -1430,9 +1436,6 @@ static pf_handle *aux_handle(pf_handle *h) {
     return h->aux;
 }
 
-// Device bytes of the two probes' Lanczos runs, their bases and a few vectors each.
-static double probe_bytes(int64_t D, int maxdim) { return 2.0 * 8.0 * (double)D * (std::min<double>(maxdim, (double)D) + 8.0); }
-
 static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, double tol, double eigentol, double *Emin,
                                 double *Emax, int *qr_restarts = nullptr, bool host_qr = false,
                                 ListRef lr = {}) {
@@ -1442,7 +1445,7 @@ static void extrema_from_device(pf_op *op, const double *v0_dev, int maxdim, dou
     if (pinned_step(op, 1, (int)sizeof(double))) {
         list = nullptr;   // the step the caller chose
     } else if (lr.own) {
-        own_list.make(op, op->h->stream, probe_bytes(D, maxdim));
+        own_list.make(op, op->h->stream);
         list = own_list.get();
     }
     // The :SR probe runs here and the :LR probe at the same time on the
@@ -1516,7 +1519,9 @@ void lanczos_extrema(pf_op *op, const double *x0_host, int maxdim, double tol, d
     AllocStream alloc_guard(op->h->stream);
     DevArray<double> v0(D);
     PF_CUDA(cudaMemcpyAsync(v0.p, seed.data(), D * sizeof(double), cudaMemcpyHostToDevice, op->h->stream));
-    extrema_from_device(op, v0.p, maxdim, tol, eigentol, Emin, Emax);
+    without_list_on_nomem(op, [&](ListRef lr) {
+        extrema_from_device(op, v0.p, maxdim, tol, eigentol, Emin, Emax, nullptr, false, lr);
+    });
 }
 
 // ------------------------------------------- op-level tensor-core Gram product
@@ -1716,9 +1721,8 @@ static bool prepare_initial_state_device(pf_op *op, int s, double *X) {
     return true;
 }
 
-void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int x0_mem, double *vals, double *vecs,
-           int vecs_mem, pf_report *rep, int *nconv) {
-    PF_CHECK(op && P && x0 && vals && nconv, PF_ERR_INVALID, "null argument");
+static void solve_with(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int x0_mem, double *vals,
+                       double *vecs, int vecs_mem, pf_report *rep, int *nconv, ListRef lr) {
     PF_CHECK(s >= 1 && nev >= 1, PF_ERR_INVALID, "s and nev must be positive");
     PF_CHECK(P->precision == PF_PREC_FP64 || P->precision == PF_PREC_MIXED, PF_ERR_INVALID, "unknown precision");
     PF_CHECK(P->reorth_passes >= 1 && P->reorth_passes <= 3, PF_ERR_INVALID, "reorth_passes must be 1, 2 or 3");
@@ -1758,11 +1762,10 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
     }
 
     // a chain's flips are listed once for the whole solve (its probes, its
-    // moments and its filter), if the rest of the solve still fits beside the list
+    // moments and its filter), or not at all
     ChainList chain_list;
+    if (lr.own) chain_list.make(op, st);
     const int probe_dim = P->extrema_maxdim > 0 ? P->extrema_maxdim : 1000;
-    chain_list.make(op, st, solve_footprint(op, P, s, nev) - (double)chain_list_bytes(op) +
-                                (P->has_Emin && P->has_Emax ? 0.0 : probe_bytes(D, probe_dim) / 2));
     const ListRef list{chain_list.get(), false};
 
     // mapping plan (Plan.jl:128-191)
@@ -1978,6 +1981,14 @@ void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int 
         R.qr_restarts += out.qr_restarts;
         *rep = R;
     }
+}
+
+void solve(pf_op *op, const pf_params *P, int s, int nev, const double *x0, int x0_mem, double *vals, double *vecs,
+           int vecs_mem, pf_report *rep, int *nconv) {
+    PF_CHECK(op && P && x0 && vals && nconv, PF_ERR_INVALID, "null argument");
+    without_list_on_nomem(op, [&](ListRef lr) {
+        solve_with(op, P, s, nev, x0, x0_mem, vals, vecs, vecs_mem, rep, nconv, lr);
+    });
 }
 
 // ------------------------------------------------ complex Hermitian input
