@@ -889,7 +889,7 @@ static double list_terms(const pf_op *op) {
 // us as for qsun_plan.  Chains (measured): 0.18 ns a row and entry in one CTA,
 // 0.27 ns on several, where a quarter of the entries are remote; wider chunks
 // cost a quarter more; 0.4 and 1.2 us for the barrier and latencies.
-// CSR rows may have their entries anywhere.  Measured over 41 matrices of 200 to
+// CSR rows may have their entries anywhere.  Measured over 40 matrices of 200 to
 // 50000 rows (chains, grids, bands, random columns; 3 to 60 entries a row), on
 // several CTAs: 1.3 ns a sector of remote columns, 0.8 ns a row, 0.38 us for each
 // eight entries of a row that wait for remote ones, as much for each eight read
@@ -1064,9 +1064,10 @@ static bool kpm_launch(ResPlan *p, int64_t D, int elem, int ncol, int M, int res
 // Of the cluster sizes and widths that fit, the one with the least estimated
 // time for all columns: as many rounds of clusters as are not resident at once,
 // or the SMs' total work where that is more.  K: a filter's order, a KPM run's steps.
-// A CSR matrix has to be ahead by 6 %: of 880 measured filters and KPM runs, the
-// choice then was slower than the step kernels in 4, by 20 % at most (by a model
-// without its columns' places: in 99, by up to a factor of 9).
+// A CSR matrix has to be ahead by 6 %: of 880 filters and KPM runs whose forms were
+// all measured, the choice then is more than 5 % slower than the step kernels in
+// 5, by 24 % at most (by a model without its columns' places in 183, by up to a
+// factor of 9.6).
 template <typename T>
 bool resident_plan(const pf_op *op, int ncol, bool kpm, int K, bool tuned, ResPlan *best) {
     const double sms = op->h->num_sms;
