@@ -21,6 +21,8 @@ def kernels(torch, call):
         call()
         torch.cuda.synchronize()
     names = {e.name for e in prof.events()}
+    if not any("(" in n for n in names):
+        pytest.skip("the profiler records no kernels here (another tool holds the device's activity records)")
     assert any("pf::" in n for n in names), names
     return names
 
